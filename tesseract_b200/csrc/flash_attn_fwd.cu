@@ -706,14 +706,20 @@ flash_bounded_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 //                   Heads of 128: one issuer for both stages. It takes them in turns, which keeps their softmaxes apart; with an
 //                   issuer each they fall into step and wait together (16384 tokens: 2.16 against 1.80 ms). Heads of 64, whose
 //                   next scores are there early: an issuer each, so that neither waits for the other's softmax (92 -> 83 us below).
-// O accumulates in TMEM over all key tiles. It is rescaled, by the softmax warps themselves, only when a row's maximum has grown
-// by more than 2^8 since the maximum that its exponents refer to was set: rarely after the first tile.
-// Per pair of tiles the exponentials take as long as the MMAs (128 x 128 of them at 16 per clock against 2 x 128^3 MACs at
-// 4096 per clock), so every instruction beside them is packed (f32x2) or left out. Measured against one tile per CTA with P in
-// shared memory and O in registers, which this kernel replaced (32 / 8 heads of 128, causal): 2 x 4096 tokens 588 -> 270 us
-// (1020 TFLOP/s), 16384 tokens 4.79 -> 1.80 ms (1220 TFLOP/s, near the sustained rate of a plain GEMM under the power limit),
-// 2 x 512 queries over 4608 keys 152 -> 84 us; 16 heads of 64, 4 x 1500 tokens, full: 177 -> 84 us (there the exponentials take
-// twice as long as the MMAs). Every fourth exponential as a polynomial on the FMA units was slower (16384 tokens: 1.92 ms).
+// O accumulates in TMEM over all key tiles and exponents refer to a row's running maximum, so that the largest probability of a row
+// is 1 and exact in bf16. (With a reference that may stay up to 2^8 behind, O need hardly ever be rescaled, but the largest
+// probability is rounded like the others: error of O before its own rounding with scores three / six times as wide as unit ones 0.0006 /
+// 0.0004 -> 0.0015 / 0.0012.) Where the maximum of any row of a warp has grown, the warp rescales O 16 columns at a time between the
+// exponentials of the first 64 keys, which hide the way to TMEM and back: by itself in front of them 0 - 14 % more with heads of 64.
+// Tiles that are masked sum the rounded probabilities, as few of them may make up a row.
+//
+// A pair of tiles takes about 3800 clocks per 128 keys, 2048 of them MMAs: a stage's softmax and its MMAs follow one another and two
+// stages fill TMEM, so every instruction of the softmax is packed (f32x2) or left out. With heads of 64 the exponentials (16 per
+// clock) take twice as long as the MMAs; with heads of 128 leaving them out changes 2 %. Measured against one tile per CTA with P in
+// shared memory and O in registers, which this kernel replaced (32 / 8 heads of 128, causal): 2 x 4096 tokens 563 -> 288 us (950
+// TFLOP/s), 16384 tokens 4.07 -> 1.97 ms (1120 TFLOP/s), 2 x 512 queries over 4608 keys 153 -> 81 us; 16 heads of 64, 4 x 1500 tokens,
+// full: 162 -> 78 us (reference up to 2^8 behind: 262 us, 1.83 ms, 78, 76 us). Every fourth exponential as a polynomial on
+// the FMA units was slower (16384 tokens: 1.80 -> 1.92 ms).
 constexpr int kPairThreads = 384;
 // Registers per thread: 168 at the launch, 208 for the softmax warps and 88 for the rest after it (256 x 208 + 128 x 88 = 384 x 168).
 constexpr int kPairSoftmaxRegs = 208, kPairOtherRegs = 88;
@@ -913,7 +919,6 @@ flash_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     const int row_limit = qi + offset;                            // last visible key under causal masking
     float m_ref = -INFINITY;                                      // the maximum that the exponents of this row refer to
     float2 l2a = make_float2(0.f, 0.f), l2b = l2a;
-    const float kGrow = 8.f;                                      // rescale when the maximum has grown by more than 2^8
     const float2 mul = both(p.scale_log2);
     bool ok = true;
     for (int j = 0; j < n_own; ++j) {
@@ -955,45 +960,55 @@ flash_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           tc_fence_after();
         }
         const bool fresh = m_ref == -INFINITY;                     // no visible scores of this row yet: O and l hold nothing of it
-        if (fresh) m_ref = m_tile;
-        const bool grow = !fresh && m_tile != -INFINITY && (m_tile - m_ref) * p.scale_log2 > kGrow;
-        if (__any_sync(0xffffffffu, grow)) {
-          // warp-collective: every lane rescales its own TMEM lane (factor 1 where nothing changed)
-          const float factor = grow ? exp2f((m_ref - m_tile) * p.scale_log2) : 1.f;
-          if (grow) m_ref = m_tile;
-#pragma unroll 1
-          for (int c = 0; c < D / 16; ++c) {
-            uint32_t r[16];
-            tmem_ld_32x16(o_addr + c * 16, r);
-            tmem_ld_wait();
+        const bool grow = m_tile > m_ref;
+        const float factor = grow && !fresh ? exp2f((m_ref - m_tile) * p.scale_log2) : 1.f;
+        if (grow) m_ref = m_tile;
+        const float2 base = both(m_ref == -INFINITY ? 0.f : -m_ref * p.scale_log2);
+        auto probabilities = [&](auto rescale) {
+          constexpr bool kRescale = decltype(rescale)::value;
 #pragma unroll
-            for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * factor);
-            tmem_st_32x16(o_addr + c * 16, r);
+          for (int c = 0; c < BKV / 64; ++c) {
+            uint32_t packed[32];
+            uint32_t r[16];
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              constexpr int kEvery = 32 / (D / 16);                // pairs of exponentials per 16 columns of O
+              if (kRescale && c == 0 && i % kEvery == 0) tmem_ld_32x16(o_addr + i / kEvery * 16, r);
+              const int e = c * 64 + 2 * i;
+              const float2 t = fma_f32x2(make_float2(__uint_as_float(sr[e]), __uint_as_float(sr[e + 1])), mul, base);
+              float2 x = make_float2(exp2_ftz(t.x), exp2_ftz(t.y));
+              if constexpr (kMask) {
+                if (e >= vis) x.x = 0.f;
+                if (e + 1 >= vis) x.y = 0.f;
+              }
+              packed[i] = pack_bf16x2(x.x, x.y);
+              if constexpr (kMask) x = make_float2(__uint_as_float(packed[i] << 16), __uint_as_float(packed[i] & 0xffff0000u));
+              if (i & 1) l2b = add_f32x2(l2b, x);
+              else l2a = add_f32x2(l2a, x);
+              if (kRescale && c == 0 && i % kEvery == kEvery - 1) {
+                tmem_ld_wait();
+#pragma unroll
+                for (int n = 0; n < 16; n += 2) {
+                  const float2 o = mul_f32x2(make_float2(__uint_as_float(r[n]), __uint_as_float(r[n + 1])), both(factor));
+                  r[n] = __float_as_uint(o.x);
+                  r[n + 1] = __float_as_uint(o.y);
+                }
+                tmem_st_32x16(o_addr + i / kEvery * 16, r);
+              }
+            }
+            tmem_st_32x32(p_addr + c * 32, packed);
+            tmem_st_wait();
+            tc_fence_before();
+            mbar_arrive(c ? &p_full[s] : &p_half[s]);
           }
+        };
+        // warp-collective: every lane rescales its own TMEM lane (factor 1 where nothing changed)
+        if (j > 0 && __any_sync(0xffffffffu, grow && !fresh)) {
           l2a = mul_f32x2(l2a, both(factor));
           l2b = mul_f32x2(l2b, both(factor));
-        }
-        const float2 base = both(m_ref == -INFINITY ? 0.f : -m_ref * p.scale_log2);
-#pragma unroll
-        for (int c = 0; c < BKV / 64; ++c) {
-          uint32_t packed[32];
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int e = c * 64 + 2 * i;
-            const float2 t = fma_f32x2(make_float2(__uint_as_float(sr[e]), __uint_as_float(sr[e + 1])), mul, base);
-            float2 x = make_float2(exp2_ftz(t.x), exp2_ftz(t.y));
-            if constexpr (kMask) {
-              if (e >= vis) x.x = 0.f;
-              if (e + 1 >= vis) x.y = 0.f;
-            }
-            if (i & 1) l2b = add_f32x2(l2b, x);
-            else l2a = add_f32x2(l2a, x);
-            packed[i] = pack_bf16x2(x.x, x.y);
-          }
-          tmem_st_32x32(p_addr + c * 32, packed);
-          tmem_st_wait();
-          tc_fence_before();
-          mbar_arrive(c ? &p_full[s] : &p_half[s]);
+          probabilities(std::true_type{});
+        } else {
+          probabilities(std::false_type{});
         }
         return true;
       };

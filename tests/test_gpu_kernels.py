@@ -317,6 +317,63 @@ def test_flash_forward_with_growing_row_maxima(dev, causal):
     assert _rel_err(got, ref) < 2e-2
 
 
+def _online_softmax(q, k, v, causal):
+    """softmax(q k^T / sqrt D) v of one head (q [Sq, D], k and v [Sk, D] in bf16) with the roundings that the kernel may make: key
+    tiles of 128, exponents relative to the running maximum, P rounded to bf16; sums in fp32, those of masked tiles of the rounded P."""
+    (Sq, D), Sk = q.shape, k.shape[0]
+    s = q.float() @ k.float().t() * D ** -0.5
+    row = torch.arange(Sq, device=q.device)[:, None] + Sk - Sq
+    if causal:
+        s = s.masked_fill(torch.arange(Sk, device=q.device) > row, float("-inf"))
+    m, l, o = torch.full((Sq, 1), float("-inf"), device=q.device), 0.0, 0.0
+    for t in range(0, Sk, 128):
+        st = s[:, t:t + 128]
+        top = torch.maximum(m, st.amax(1, keepdim=True))
+        base = top.masked_fill(top == float("-inf"), 0.0)
+        p = torch.exp(st - base)
+        first = torch.arange(Sq, device=q.device)[:, None] // 128 * 128 + Sk - Sq         # position of the query tile's first row
+        masked = (t + 127 > first) if causal else torch.full_like(row, t + 128 > Sk, dtype=torch.bool)
+        f = torch.exp(m - base)
+        l = l * f + torch.where(masked, p.bfloat16().float(), p).sum(1, keepdim=True)
+        o, m = o * f + p.bfloat16().float() @ v[t:t + 128].float(), top
+    return o / l, m - s[:, :128].amax(1, keepdim=True)
+
+
+@pytest.mark.parametrize("H,Hkv", [(4, 2), (3, 3)])               # two heads of a group per CTA; two tiles of a head
+@pytest.mark.parametrize("Sq,Sk", [(700, 700), (300, 1200)])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("width,grow", [(1.0, False), (3.0, False), (6.0, False), (1.0, True)])
+def test_flash_forward_accuracy_over_score_widths(dev, H, Hkv, Sq, Sk, D, width, grow):
+    """Scores of unit width, as wide as in trained models, and growing along the keys by more than 2^8 at a time: no further from 64
+    bits than the arithmetic above (5 % for the order of sums and the exponential's last bits), whatever the output's scale in TMEM."""
+    from tesseract_b200.ops import flash_attention
+    g = torch.Generator(device=dev).manual_seed(Sq + D)
+    q = (torch.randn(1, Sq, H, D, device=dev, generator=g) * width).bfloat16()
+    k = torch.randn(1, Sk, Hkv, D, device=dev, generator=g)
+    if grow:
+        k = k * torch.linspace(0.2, 12.0, Sk, device=dev).view(1, Sk, 1, 1)
+    k, v = k.bfloat16(), torch.randn(1, Sk, Hkv, D, device=dev, generator=g).bfloat16()
+    for causal in (True, False):
+        with torch.no_grad():
+            got = flash_attention(q, k, v, causal=causal)
+        torch.cuda.synchronize()
+        _status_ok()
+        worst, mine, theirs, norm = 0.0, 0.0, 0.0, 0.0
+        for h in range(H):
+            qh, kh, vh = q[0, :, h], k[0, :, h // (H // Hkv)], v[0, :, h // (H // Hkv)]
+            s = qh.double() @ kh.double().t() * D ** -0.5
+            if causal:
+                s = s.masked_fill(torch.arange(Sk, device=dev) > torch.arange(Sq, device=dev)[:, None] + Sk - Sq, float("-inf"))
+            ref = torch.softmax(s, -1) @ vh.double()
+            o, rise = _online_softmax(qh, kh, vh, causal)
+            worst = max(worst, float(rise.max()))
+            mine += float((got[0, :, h].double() - ref).square().sum())
+            theirs += float((o.bfloat16().double() - ref).square().sum())
+            norm += float(ref.square().sum())
+        assert not grow or worst > 8.0                             # (in units of e: more than 2^8 after the first 128 keys)
+        assert mine <= theirs * 1.05 ** 2, ((mine / norm) ** 0.5, (theirs / norm) ** 0.5)
+
+
 @pytest.mark.parametrize("M", [1, 2, 3, 4])
 @pytest.mark.parametrize("N,K", [(1, 16), (7, 272), (149, 4096), (2049, 528), (33, 24576), (1000, 1040)])
 @pytest.mark.parametrize("pdl", [False, True])
