@@ -105,9 +105,10 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  // KV heads on the fast axis: under causal masking the first key tiles, seen by the most queries, all start first
-  const int hk = blockIdx.x;
-  const int j = blockIdx.y;  // key tile
+  // KV heads on the fast axis: under causal masking the first key tiles, seen by the most queries, all start first. (Both on x: key
+  // tiles may be more than the other axes take.)
+  const int j = blockIdx.x / p.Hkv;  // key tile
+  const int hk = blockIdx.x - j * p.Hkv;
   const int b = blockIdx.z;
   const int G = p.H / p.Hkv;
   const int c0 = j * BT;
@@ -547,7 +548,7 @@ TSB_EXPORT int tsb_flash_bwd(const void* dO, const void* q, const void* k, const
     if (e != cudaSuccess) return static_cast<int>(e);
     rows_kern<<<static_cast<unsigned>((rows * (kD / 8) + 255) / 256), 256, 0, s>>>(
         static_cast<const __nv_bfloat16*>(dO), static_cast<const __nv_bfloat16*>(o), lse, lse2, delta, dq_acc, rows, Sq, n_q * BT, H);
-    kern<<<dim3(Hkv, (Sk + BT - 1) / BT, B), kBwdThreads, BwdCfg<kD>::kSmemBytes, s>>>(tq, tk, tv, tdo, p);
+    kern<<<dim3(static_cast<unsigned>(Hkv) * ((Sk + BT - 1) / BT), 1, B), kBwdThreads, BwdCfg<kD>::kSmemBytes, s>>>(tq, tk, tv, tdo, p);
     e = cudaGetLastError();
     if (e != cudaSuccess) return static_cast<int>(e);
     dq_kern<<<dim3(n_q, H, B), 128, 0, s>>>(dq_acc, static_cast<__nv_bfloat16*>(dq), scale, H, Sq, g_sb, g_ss, g_sh);

@@ -754,11 +754,12 @@ flash_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     }
     bb = 0;
   }
-  // heads on the fast axis, late (heavy) query tiles first: the last CTAs to start are the lightest ones
-  const int qt = gridDim.y - 1 - blockIdx.y;
+  // heads on the fast axis, late (heavy) query tiles first: the last CTAs to start are the lightest ones. (Both on x: tiles of a
+  // long sequence may be more than the other axes take.)
+  const int heads = pair_heads ? p.H / 2 : p.H, tile = blockIdx.x / heads, qt = gridDim.x / heads - 1 - tile;
   const int qa = pair_heads ? qt * BQ : qt * 2 * BQ;              // first query row of stage 0
   if (qa >= Sq) return;
-  const int ha = pair_heads ? blockIdx.x * 2 : blockIdx.x;
+  const int ha = (blockIdx.x - tile * heads) * (pair_heads ? 2 : 1);
   const int hk = ha / (p.H / p.Hkv), offset = Sk - Sq;
   int n_of[2];                               // key tiles of each stage
 #pragma unroll
@@ -1075,7 +1076,7 @@ flash_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 // p.Sq: the query rows (of the longest sequence).
 int launch_pair(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaParams& p, int D, cudaStream_t stream) {
   const int pair_heads = (p.H / p.Hkv) % 2 == 0, rows = pair_heads ? BQ : 2 * BQ;
-  const dim3 grid(pair_heads ? p.H / 2 : p.H, (p.Sq + rows - 1) / rows, p.B);
+  const dim3 grid(static_cast<unsigned>(pair_heads ? p.H / 2 : p.H) * ((p.Sq + rows - 1) / rows), 1, p.B);
   auto go = [&](auto kern, int smem_bytes) -> int {
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
     if (e != cudaSuccess) return static_cast<int>(e);

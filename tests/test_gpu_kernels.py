@@ -591,6 +591,42 @@ def test_flash_backward_tile_edges(dev, H, Hkv, Sq, Sk, D):
             assert _rel_err(a, b) < 6e-3, (name, causal)
 
 
+@pytest.mark.parametrize("H,Hkv,Sq", [(2, 1, 65535 * 128 + 20), (1, 1, 65535 * 256 + 20)])
+def test_flash_forward_more_tiles_than_a_short_grid_axis(dev, H, Hkv, Sq):
+    """More query tiles than the y axis of a grid takes. Rows at both ends: 0.0017 of a row, as for the tiles' edges below."""
+    from tesseract_b200 import ops
+    g = torch.Generator(device=dev).manual_seed(3)
+    q = torch.randn(1, Sq, H, 64, device=dev, generator=g, dtype=torch.bfloat16)
+    k, v = (torch.randn(1, 48, Hkv, 64, device=dev, generator=g, dtype=torch.bfloat16) for _ in range(2))
+    with torch.no_grad():
+        o = ops.flash_attention(q, k, v, causal=False)
+    torch.cuda.synchronize()
+    _status_ok()
+    for rows in (slice(0, 300), slice(Sq - 300, Sq)):
+        ref = ops.attention_ref(q[:, rows].transpose(1, 2).float(), k.transpose(1, 2).float(), v.transpose(1, 2).float(), causal=False)
+        assert _rel_err(o[:, rows], ref.transpose(1, 2)) < 5e-3
+
+
+def test_flash_backward_more_tiles_than_a_short_grid_axis(dev):
+    """More key tiles than the y axis of a grid takes, a tile's part of queries. Gradients as above: about 0.002 of a row."""
+    from tesseract_b200 import ops
+    Sq, Sk = 16, 65535 * 128 + 20
+    g = torch.Generator(device=dev).manual_seed(4)
+    q = torch.randn(1, Sq, 1, 64, device=dev, generator=g, dtype=torch.bfloat16).requires_grad_()
+    k, v = (torch.randn(1, Sk, 1, 64, device=dev, generator=g, dtype=torch.bfloat16).requires_grad_() for _ in range(2))
+    do = torch.randn(1, Sq, 1, 64, device=dev, generator=g, dtype=torch.bfloat16)
+    got = torch.autograd.grad(ops.flash_attention(q, k, v, causal=False), (q, k, v), do)
+    torch.cuda.synchronize()
+    _status_ok()
+    qf, kf, vf, df = (t.detach()[0, :, 0].float() for t in (q, k, v, do))
+    p = torch.softmax(qf @ kf.t() / 8.0, -1)
+    dp = df @ vf.t()
+    ds = p * (dp - (p * dp).sum(1, keepdim=True)) / 8.0
+    for name, a, b in zip("qkv", got, (ds @ kf, ds.t() @ qf, p.t() @ df)):
+        for rows in (slice(0, 300), slice(-300, None)):
+            assert _rel_err(a[0, rows, 0], b[rows]) < 6e-3, name
+
+
 def _make_paged(dev, A, Hkv, D, bs, lens, dtype, int8):
     from tesseract_b200.nn.kv_cache import quantize_kv_per_token
     nb = sum((l + bs - 1) // bs for l in lens) + 3
