@@ -739,10 +739,17 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   return d;
 }
 
+// The two tiles of a CTA: neighbouring tiles of a head, the same tile of two heads, or one tile alone. Alone where all tiles together
+// are at most one per SM: two of them on an SM wait for each other's MMAs and issue slots, and the other SM idles. One / two per CTA in
+// us (one tile per CTA of the kernel before): 8 heads of 128, 128 queries over 8192 keys 119 / 134 (129); 16 heads, 512 over 4608 72 / 80
+// (77); 4 heads, 1000 causal 22 / 27 (23); 32 heads of 64, 256 over 4096 47 / 58 (66). With more tiles than SMs, two per CTA cost less
+// than a second round of CTAs.
+enum class PairOf { kTiles, kHeads, kOne };
+
 template <int D>
 __global__ void __launch_bounds__(kPairThreads, 1)
 flash_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                  const __grid_constant__ CUtensorMap tmV, FaParams p, int pair_heads) {
+                  const __grid_constant__ CUtensorMap tmV, FaParams p, PairOf pair) {
   using Cfg = PairCfg<D>;
   int Sq = p.Sq, Sk = p.Sk, row0 = 0, krow0 = 0, bb = blockIdx.z;
   if (p.cu_seqlens) {                        // sequences one after another on one token axis (tensor maps with batch 1)
@@ -756,8 +763,9 @@ flash_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   }
   // heads on the fast axis, late (heavy) query tiles first: the last CTAs to start are the lightest ones. (Both on x: tiles of a
   // long sequence may be more than the other axes take.)
+  const bool pair_heads = pair == PairOf::kHeads;
   const int heads = pair_heads ? p.H / 2 : p.H, tile = blockIdx.x / heads, qt = gridDim.x / heads - 1 - tile;
-  const int qa = pair_heads ? qt * BQ : qt * 2 * BQ;              // first query row of stage 0
+  const int qa = pair == PairOf::kTiles ? qt * 2 * BQ : qt * BQ;  // first query row of stage 0
   if (qa >= Sq) return;
   const int ha = (blockIdx.x - tile * heads) * (pair_heads ? 2 : 1);
   const int hk = ha / (p.H / p.Hkv), offset = Sk - Sq;
@@ -770,7 +778,7 @@ flash_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       const int last = q0 + BQ - 1 + offset;
       n = min(n, last < 0 ? 0 : last / BKV + 1);
     }
-    n_of[s] = q0 < Sq ? n : 0;
+    n_of[s] = q0 < Sq && !(s && pair == PairOf::kOne) ? n : 0;
   }
   const int n_tiles = max(n_of[0], n_of[1]);
 
@@ -1022,7 +1030,7 @@ flash_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     bool have = ok && n_own > 0;
     if (have) have = mbar_wait(&o_full[s], Cfg::kOwnP ? (n_own - 1) & 1 : 0, &cta_abort, p.status);
     have = __all_sync(0xffffffffu, have ? 1 : 0) != 0;
-    if (have || (n_own == 0 && q0 < Sq)) {
+    if (have || (n_own == 0 && q0 < Sq && !(s && pair == PairOf::kOne))) {
       if (have) tc_fence_after();
       const float l = (l2a.x + l2a.y) + (l2b.x + l2b.y), inv_l = l > 0.f ? 1.f / l : 0.f;
       // Q of this stage is not needed any more: its shared memory turns the rows, so that a warp stores whole rows
@@ -1075,12 +1083,14 @@ flash_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 
 // p.Sq: the query rows (of the longest sequence).
 int launch_pair(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaParams& p, int D, cudaStream_t stream) {
-  const int pair_heads = (p.H / p.Hkv) % 2 == 0, rows = pair_heads ? BQ : 2 * BQ;
-  const dim3 grid(static_cast<unsigned>(pair_heads ? p.H / 2 : p.H) * ((p.Sq + rows - 1) / rows), 1, p.B);
+  const long long tiles = (p.Sq + BQ - 1) / BQ, all = tiles * p.H * p.B;
+  const PairOf pair = all <= sm_count() ? PairOf::kOne : (p.H / p.Hkv) % 2 == 0 ? PairOf::kHeads : PairOf::kTiles;
+  const dim3 grid(static_cast<unsigned>(pair == PairOf::kOne ? tiles * p.H : pair == PairOf::kHeads ? tiles * (p.H / 2) : (tiles + 1) / 2 * p.H),
+                  1, p.B);
   auto go = [&](auto kern, int smem_bytes) -> int {
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
     if (e != cudaSuccess) return static_cast<int>(e);
-    kern<<<grid, kPairThreads, smem_bytes, stream>>>(tq, tk, tv, p, pair_heads);
+    kern<<<grid, kPairThreads, smem_bytes, stream>>>(tq, tk, tv, p, pair);
     return static_cast<int>(cudaGetLastError());
   };
   return D == 128 ? go(flash_pair_kernel<128>, PairCfg<128>::kSmemBytes) : go(flash_pair_kernel<64>, PairCfg<64>::kSmemBytes);

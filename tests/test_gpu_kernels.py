@@ -318,60 +318,55 @@ def test_flash_forward_with_growing_row_maxima(dev, causal):
 
 
 def _online_softmax(q, k, v, causal):
-    """softmax(q k^T / sqrt D) v of one head (q [Sq, D], k and v [Sk, D] in bf16) with the roundings that the kernel may make: key
-    tiles of 128, exponents relative to the running maximum, P rounded to bf16; sums in fp32, those of masked tiles of the rounded P."""
-    (Sq, D), Sk = q.shape, k.shape[0]
-    s = q.float() @ k.float().t() * D ** -0.5
+    """softmax(q k^T / sqrt D) v of heads (q [N, Sq, D], k and v [N, Sk, D] in bf16) with the roundings that the kernel may make: key
+    tiles of 128, exponents relative to the running maximum, P rounded to bf16; sums in fp32, those of masked tiles of the rounded P.
+    Also by how much the rows' maxima rise after the first 128 keys."""
+    (N, Sq, D), Sk = q.shape, k.shape[1]
+    s = q.float() @ k.float().transpose(1, 2) * D ** -0.5
     row = torch.arange(Sq, device=q.device)[:, None] + Sk - Sq
     if causal:
         s = s.masked_fill(torch.arange(Sk, device=q.device) > row, float("-inf"))
-    m, l, o = torch.full((Sq, 1), float("-inf"), device=q.device), 0.0, 0.0
+    first = torch.arange(Sq, device=q.device)[:, None] // 128 * 128 + Sk - Sq             # position of the query tile's first row
+    m, l, o = torch.full((N, Sq, 1), float("-inf"), device=q.device), 0.0, 0.0
     for t in range(0, Sk, 128):
-        st = s[:, t:t + 128]
-        top = torch.maximum(m, st.amax(1, keepdim=True))
+        st = s[:, :, t:t + 128]
+        top = torch.maximum(m, st.amax(2, keepdim=True))
         base = top.masked_fill(top == float("-inf"), 0.0)
-        p = torch.exp(st - base)
-        first = torch.arange(Sq, device=q.device)[:, None] // 128 * 128 + Sk - Sq         # position of the query tile's first row
+        p, f = torch.exp(st - base), torch.exp(m - base)
         masked = (t + 127 > first) if causal else torch.full_like(row, t + 128 > Sk, dtype=torch.bool)
-        f = torch.exp(m - base)
-        l = l * f + torch.where(masked, p.bfloat16().float(), p).sum(1, keepdim=True)
-        o, m = o * f + p.bfloat16().float() @ v[t:t + 128].float(), top
-    return o / l, m - s[:, :128].amax(1, keepdim=True)
+        l = l * f + torch.where(masked, p.bfloat16().float(), p).sum(2, keepdim=True)
+        o, m = o * f + p.bfloat16().float() @ v[:, t:t + 128].float(), top
+    return o / l, m - s[:, :, :128].amax(2, keepdim=True)
 
 
-@pytest.mark.parametrize("H,Hkv", [(4, 2), (3, 3)])               # two heads of a group per CTA; two tiles of a head
+@pytest.mark.parametrize("B,H,Hkv", [(1, 4, 2), (20, 4, 2), (20, 3, 3)])      # a tile per CTA; two heads of a group; two tiles of a head
 @pytest.mark.parametrize("Sq,Sk", [(700, 700), (300, 1200)])
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("width,grow", [(1.0, False), (3.0, False), (6.0, False), (1.0, True)])
-def test_flash_forward_accuracy_over_score_widths(dev, H, Hkv, Sq, Sk, D, width, grow):
+def test_flash_forward_accuracy_over_score_widths(dev, B, H, Hkv, Sq, Sk, D, width, grow):
     """Scores of unit width, as wide as in trained models, and growing along the keys by more than 2^8 at a time: no further from 64
     bits than the arithmetic above (5 % for the order of sums and the exponential's last bits), whatever the output's scale in TMEM."""
     from tesseract_b200.ops import flash_attention
     g = torch.Generator(device=dev).manual_seed(Sq + D)
-    q = (torch.randn(1, Sq, H, D, device=dev, generator=g) * width).bfloat16()
-    k = torch.randn(1, Sk, Hkv, D, device=dev, generator=g)
+    q = (torch.randn(B, Sq, H, D, device=dev, generator=g) * width).bfloat16()
+    k = torch.randn(B, Sk, Hkv, D, device=dev, generator=g)
     if grow:
         k = k * torch.linspace(0.2, 12.0, Sk, device=dev).view(1, Sk, 1, 1)
-    k, v = k.bfloat16(), torch.randn(1, Sk, Hkv, D, device=dev, generator=g).bfloat16()
+    k, v = k.bfloat16(), torch.randn(B, Sk, Hkv, D, device=dev, generator=g).bfloat16()
+    rows = [t.repeat_interleave(n, 2).transpose(1, 2).flatten(0, 1) for t, n in ((q, 1), (k, H // Hkv), (v, H // Hkv))]
     for causal in (True, False):
         with torch.no_grad():
-            got = flash_attention(q, k, v, causal=causal)
+            got = flash_attention(q, k, v, causal=causal).transpose(1, 2).flatten(0, 1)
         torch.cuda.synchronize()
         _status_ok()
-        worst, mine, theirs, norm = 0.0, 0.0, 0.0, 0.0
-        for h in range(H):
-            qh, kh, vh = q[0, :, h], k[0, :, h // (H // Hkv)], v[0, :, h // (H // Hkv)]
-            s = qh.double() @ kh.double().t() * D ** -0.5
-            if causal:
-                s = s.masked_fill(torch.arange(Sk, device=dev) > torch.arange(Sq, device=dev)[:, None] + Sk - Sq, float("-inf"))
-            ref = torch.softmax(s, -1) @ vh.double()
-            o, rise = _online_softmax(qh, kh, vh, causal)
-            worst = max(worst, float(rise.max()))
-            mine += float((got[0, :, h].double() - ref).square().sum())
-            theirs += float((o.bfloat16().double() - ref).square().sum())
-            norm += float(ref.square().sum())
-        assert not grow or worst > 8.0                             # (in units of e: more than 2^8 after the first 128 keys)
-        assert mine <= theirs * 1.05 ** 2, ((mine / norm) ** 0.5, (theirs / norm) ** 0.5)
+        s = rows[0].double() @ rows[1].double().transpose(1, 2) * D ** -0.5
+        if causal:
+            s = s.masked_fill(torch.arange(Sk, device=dev) > torch.arange(Sq, device=dev)[:, None] + Sk - Sq, float("-inf"))
+        ref = torch.softmax(s, -1) @ rows[2].double()
+        o, rise = _online_softmax(*rows, causal)
+        assert not grow or float(rise.max()) > 8.0                 # (in units of e: more than 2^8)
+        mine, theirs = (float((x.double() - ref).norm() / ref.norm()) for x in (got, o.bfloat16()))
+        assert mine <= theirs * 1.05, (mine, theirs)
 
 
 @pytest.mark.parametrize("M", [1, 2, 3, 4])
@@ -412,11 +407,11 @@ def test_cluster_splitk_gemm(dev, M, N, K, split):
 
 
 @pytest.mark.parametrize("D", [128, 64])
-def test_flash_varlen_matches_per_sequence(dev, D):
+@pytest.mark.parametrize("H,Hkv,copies", [(8, 2, 1), (8, 2, 3), (9, 3, 3)])   # a tile per CTA; two heads of a group; two tiles of a head
+def test_flash_varlen_matches_per_sequence(dev, D, H, Hkv, copies):
     """Prompts of different lengths packed on one token axis, one launch, against per-sequence attention."""
     from tesseract_b200 import ops
-    H, Hkv = 8, 2
-    lens = [5, 300, 128, 1, 257, 64]
+    lens = [5, 300, 128, 1, 257, 64] * copies
     g = torch.Generator(device=dev).manual_seed(D)
     qkv = torch.randn(sum(lens), H + 2 * Hkv, D, device=dev, generator=g).bfloat16()
     cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=dev)
@@ -498,13 +493,14 @@ def test_gemm_tiles_of_two_sms(dev, M, N, K, a_mn, b_mn, out, accumulate):
 @pytest.mark.parametrize("H,Hkv", [(4, 2), (3, 3), (6, 2)])       # two heads of a group per CTA; two tiles of a head
 @pytest.mark.parametrize("Sq,Sk", [(1, 1), (1, 300), (127, 127), (128, 128), (129, 640), (257, 257), (300, 200)])
 @pytest.mark.parametrize("D", [64, 128])
-def test_flash_forward_tile_pairs(dev, H, Hkv, Sq, Sk, D):
+@pytest.mark.parametrize("B", [2, 80])                            # a tile per CTA while that fills one round of them; pairs of tiles
+def test_flash_forward_tile_pairs(dev, H, Hkv, Sq, Sk, D, B):
     """Ends of tiles and of pairs of tiles, rows without a visible key. P and the output are rounded to bf16 (each 2^-9 / sqrt 3
     of a value in the mean), so the error of a row is about 0.0017 of it; 0.005 leaves three times that."""
     from tesseract_b200 import ops
     g = torch.Generator(device=dev).manual_seed(Sq + Sk + D)
-    q = torch.randn(2, Sq, H, D, device=dev, generator=g).bfloat16()
-    k, v = (torch.randn(2, Sk, Hkv, D, device=dev, generator=g).bfloat16() for _ in range(2))
+    q = torch.randn(B, Sq, H, D, device=dev, generator=g).bfloat16()
+    k, v = (torch.randn(B, Sk, Hkv, D, device=dev, generator=g).bfloat16() for _ in range(2))
     for causal in (True, False):
         with torch.no_grad():
             o = ops.flash_attention(q, k, v, causal=causal)
