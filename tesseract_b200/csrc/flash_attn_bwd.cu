@@ -438,7 +438,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 }
 
 // Per row of [B, H, n_q * 128]: lse2 = lse * log2 e and delta = sum_d dO * O (both [B, Sq, H, D], contiguous), and the row's share
-// of the zeroes of dq_acc. D / 8 lanes take a row, 16 bytes each.
+// of the zeroes of dq_acc. D / 8 lanes take a row, 16 bytes each; an O whose base is not aligned to that is read by elements.
 template <int D>
 __global__ void __launch_bounds__(256)
 flash_bwd_rows_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __restrict__ O, const float* __restrict__ lse,
@@ -452,7 +452,14 @@ flash_bwd_rows_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16*
   float acc = 0.f;
   if (s < Sq) {
     const long long b = bh / H, src = ((b * Sq + s) * H + (bh - b * H)) * D + c * 8;
-    const uint4 x = *reinterpret_cast<const uint4*>(dO + src), y = *reinterpret_cast<const uint4*>(O + src);
+    const uint4 x = *reinterpret_cast<const uint4*>(dO + src);
+    uint4 y;
+    if ((reinterpret_cast<uintptr_t>(O) & 15) == 0) {
+      y = *reinterpret_cast<const uint4*>(O + src);
+    } else {
+      const unsigned short* e = reinterpret_cast<const unsigned short*>(O + src);
+      y = make_uint4(e[0] | e[1] << 16, e[2] | e[3] << 16, e[4] | e[5] << 16, e[6] | e[7] << 16);
+    }
     const __nv_bfloat162 *x2 = reinterpret_cast<const __nv_bfloat162*>(&x), *y2 = reinterpret_cast<const __nv_bfloat162*>(&y);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -504,7 +511,7 @@ TSB_EXPORT long long tsb_flash_bwd_scratch_bytes(int B, int Sq, int H, int D) {
   return (static_cast<long long>(B) * Sq * H * D + 2 * static_cast<long long>(B) * H * Sp) * 4;
 }
 
-// Gradients of tsb_flash_fwd. dO and O are contiguous [B, Sq, H, D]. dq / dk / dv are bf16 views that share the stride triple
+// Gradients of tsb_flash_fwd. dO and O are contiguous [B, Sq, H, D], dO, q, k and v 16-byte aligned. dq / dk / dv are bf16 views that share the stride triple
 // (g_sb, g_ss, g_sh) -- usually slices of one packed [B, S, H + 2 Hkv, D] buffer.
 // scratch: tsb_flash_bwd_scratch_bytes() bytes of device memory, 16-byte aligned (contents are overwritten).
 TSB_EXPORT int tsb_flash_bwd(const void* dO, const void* q, const void* k, const void* v, const void* o,

@@ -623,6 +623,33 @@ def test_flash_backward_more_tiles_than_a_short_grid_axis(dev):
             assert _rel_err(a[0, rows, 0], b[rows]) < 6e-3, name
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("shift", [1, 2, 4])
+def test_flash_backward_takes_an_output_at_any_address(dev, D, shift):
+    """A saved output that a hook brings back somewhere else, not aligned to 16 bytes: the same dK and dV to the last bit."""
+    from tesseract_b200 import ops
+    g = torch.Generator(device=dev).manual_seed(D)
+    q, k, v, do = (torch.randn(2, 200, 4, D, device=dev, generator=g).bfloat16() for _ in range(4))
+    q, k, v = (t.requires_grad_() for t in (q, k, v))
+    want = torch.autograd.grad(ops.flash_attention(q, k, v, causal=True), (q, k, v), do)
+    moved = []
+
+    def elsewhere(t):
+        if t.data_ptr() != o.data_ptr():
+            return t
+        moved.append(torch.empty(t.numel() + shift, device=dev, dtype=t.dtype)[shift:].view_as(t).copy_(t))
+        return moved[-1]
+
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.detach(), elsewhere):
+        o = ops.flash_attention(q, k, v, causal=True)
+    got = torch.autograd.grad(o, (q, k, v), do)
+    torch.cuda.synchronize()
+    _status_ok()
+    assert len(moved) == 1 and moved[0].data_ptr() % 16
+    assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
+    assert _rel_err(got[0], want[0].float()) < 1e-3                # (dQ is summed by atomics: a last bit of bf16 here and there)
+
+
 def _make_paged(dev, A, Hkv, D, bs, lens, dtype, int8):
     from tesseract_b200.nn.kv_cache import quantize_kv_per_token
     nb = sum((l + bs - 1) // bs for l in lens) + 3
