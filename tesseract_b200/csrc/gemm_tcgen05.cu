@@ -391,9 +391,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // The same product on tiles of 256 x 256 that a cluster of two CTAs works on together: `tcgen05.mma.cta_group::2`, issued by the first
 // CTA, multiplies the 256 rows of A (128 in each CTA's shared memory) with the 256 columns of B (128 in each), and each CTA's TMEM
 // receives its 128 rows. Against 128 x 256 tiles per CTA a CTA stages and reads a third less per product (32 instead of 48 KB per
-// 64 of K), so the ring holds six stages instead of four and, which counts under the power limit, fewer bytes move. Sustained over
-// 0.35 s, in TFLOP/s, 128 x 256 per CTA -> 256 x 256 per pair: 8192 x 28672 x 4096 1254 -> 1290, its weight gradient 1123 -> 1163, its
-// input gradient 1205 -> 1199; 8192 x 4096 x 4096 1185 -> 1215 / 1049 -> 1080 / 1171 -> 1202; 3003 x 16384 x 2048 1028 -> 1083.
+// 64 of K), so the ring holds six stages instead of four and, which counts under the power limit, fewer bytes move. What it gives depends
+// on K (tsb_gemm_bf16): below, the stores of a tile, which two SMs start together, take longer than its products.
 //   every CTA   warp 0 loads its halves of A and B; the bytes are counted on the first CTA's barrier. Warps 2-5 store its rows.
 //   first CTA   warp 1 issues the MMAs; its commits arrive in both CTAs.
 struct PairTile {
@@ -722,8 +721,11 @@ TSB_EXPORT int tsb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
     const int sms = sm_count();
     const long long mt = (M + BM - 1) / BM;
     auto tiles = [&](int b) { return mt * ((N + b - 1) / b); };
-    // 128 x 256 tiles would be chosen, and tiles of 256 x 256 for pairs of SMs take no more rounds than they
-    if (max_ctas <= 0 && N >= 256 && tiles(256) >= sms) {
+    // 128 x 256 tiles would be chosen, and tiles of 256 x 256 for pairs of SMs take no more rounds than they. Time of the former over that of
+    // the latter, sustained: K = 256 0.82, 512 0.98, 768 0.96 - 1.01, 896 0.97 - 1.07, 960 1.08, 1024 - 1536 1.00 - 1.14 (9001 x 1288 x 1000
+    // 1.21), 2048 - 8192 1.00 - 1.08 (two rounds of which the second is a third full 1.00, 8192 x 28672 x 4096 1.05), 9216 - 12288 1.00 - 1.02,
+    // beyond 0.975 - 1.01 (4096 x 4096 x 128256 0.975, 8192 x 4096 x 28672 0.985, 17408 1.007). (Runs of one side differ by 1 %.)
+    if (max_ctas <= 0 && N >= 256 && tiles(256) >= sms && K >= 960 && K <= 12288) {
       const long long pairs = sms / 2, tiles2 = ((M + 255) / 256) * static_cast<long long>((N + 255) / 256);
       pair = (tiles2 + pairs - 1) / pairs <= (tiles(256) + sms - 1) / sms;
     }

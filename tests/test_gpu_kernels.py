@@ -471,23 +471,27 @@ def test_tiny_llama_train_step_matches_cpu(dev):
     assert worst < 8e-2, worst
 
 
-@pytest.mark.parametrize("M,N,K", [(4864, 4096, 64), (4872, 4104, 520), (9000, 2312, 136)])    # whole tiles; ends of every kind
+@pytest.mark.parametrize("M,N,K,pad", [(4864, 4096, 64, 0), (4872, 4104, 520, 0), (9000, 2312, 136, 0),      # 128 x 256 tiles; from here on pairs
+                                       (4864, 4096, 960, 0), (4872, 4104, 1032, 0), (9000, 2312, 1000, 3), (4864, 4096, 12288, 0)])
 @pytest.mark.parametrize("a_mn", [False, True])
 @pytest.mark.parametrize("b_mn", [False, True])
 @pytest.mark.parametrize("out,accumulate", [(torch.bfloat16, False), (torch.bfloat16, True), (torch.float32, True)])
-def test_gemm_tiles_of_two_sms(dev, M, N, K, a_mn, b_mn, out, accumulate):
-    """Products large enough for 256 x 256 tiles. fp32 sums of exact products, in another order than the reference's: 1e-4 at most
-    at these depths; a bf16 result is rounded once more, 2^-9 / sqrt 3 = 0.0011 of it in the mean."""
+def test_gemm_tiles_of_two_sms(dev, M, N, K, pad, a_mn, b_mn, out, accumulate):
+    """Products large enough for 256 x 256 tiles: whole tiles, ends of every kind, result rows that allow no wide stores. fp32 sums
+    of exact products, in another order than the reference's: 1e-4 at most at these depths; a bf16 result is rounded once more,
+    2^-9 / sqrt 3 = 0.0011 of it in the mean."""
     from tesseract_b200.ops.gemm import gemm_bf16
     g = torch.Generator(device=dev).manual_seed(M + N + K)
     a = torch.randn(*((K, M) if a_mn else (M, K)), device=dev, generator=g).bfloat16()
     b = torch.randn(*((K, N) if b_mn else (N, K)), device=dev, generator=g).bfloat16()
-    c = torch.randn(M, N, device=dev, generator=g).to(out)
+    rows = torch.randn(M, N + pad, device=dev, generator=g).to(out)
+    beside, c = rows[:, N:].clone(), rows[:, :N]
     ref = (a.t() if a_mn else a).double() @ (b if b_mn else b.t()).double() + (c.double() if accumulate else 0)
     gemm_bf16(a, b, a_mn=a_mn, b_mn=b_mn, out=c, accumulate=accumulate)
     torch.cuda.synchronize()
     _status_ok()
     assert float((c.double() - ref).norm() / ref.norm()) < (3e-3 if out == torch.bfloat16 else 1e-4)
+    assert torch.equal(rows[:, N:], beside)
 
 
 @pytest.mark.parametrize("H,Hkv", [(4, 2), (3, 3), (6, 2)])       # two heads of a group per CTA; two tiles of a head
