@@ -195,16 +195,20 @@ rmsnorm_fwd_pf_kernel(const T* __restrict__ x, const T* __restrict__ res, const 
 // dx = rstd * (dy*w - xhat * mean(dy*w*xhat)) (+ dres);  dw partial sums per CTA into `dw_partial[grid, D]`.
 // Bound by the bytes in flight: the next row's three inputs are requested, and kept packed, before this row's sum goes through the
 // two barriers of its reduction. With the sum over the parts below, us before -> now: 8192 x 4096 bf16 102 -> 52 (5.2 TB/s),
-// 8192 x 8192 314 -> 101, 4096 x 4096 fp32 70 -> 58, 3003 x 2048 bf16 25 -> 13, 512 x 256 13 -> 6.
+// 8192 x 8192 314 -> 101, 3003 x 2048 25 -> 13, 512 x 256 13 -> 6; fp32 4096 x 4096 70 -> 52, 4096 x 8192 190 -> 123, 17 x 8192
+// 7.3 -> 6.7. fp32 has one CTA per SM from 2048 columns on: two, held to 128 registers, spilled 92 bytes (58 us at 4096 x 4096).
 template <typename T, int MAXV>
-__global__ void __launch_bounds__(256, MAXV <= 2 ? 2 : 1)
+__global__ void __launch_bounds__(256, MAXV * sizeof(T) <= 4 ? 2 : 1)
 rmsnorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ w,
                    const float* __restrict__ rstd_in, const T* __restrict__ dres, T* __restrict__ dx,
                    float* __restrict__ dw_partial, int rows, int D) {
+  // (fp32 rows of more than 4096 fill the registers: their `dres` is read where it is used. Ahead, 96 bytes spilled: 142 us at
+  // 4096 x 8192, 17 x 8192 7.7 against 7.3 before.)
+  constexpr bool kResAhead = MAXV * sizeof(T) < 16;
   __shared__ float red[32];
   const int nvec = D / 8;
   float dwacc[MAXV][8];
-  Raw8<T> wv[MAXV], nx[MAXV], ng[MAXV], nr[MAXV];
+  Raw8<T> wv[MAXV], nx[MAXV], ng[MAXV], nr[kResAhead ? MAXV : 1];
   float nrstd = 0.f;
   auto fetch = [&](int row) {
     const size_t off = static_cast<size_t>(row) * D;
@@ -215,7 +219,7 @@ rmsnorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* _
       if (v < nvec) {
         nx[i] = ldraw8<T>(x + off + v * 8);
         ng[i] = ldraw8<T>(dy + off + v * 8);
-        if (dres) nr[i] = ldraw8<T>(dres + off + v * 8);
+        if (kResAhead && dres) nr[i] = ldraw8<T>(dres + off + v * 8);
       }
     }
   };
@@ -232,7 +236,7 @@ rmsnorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* _
     const size_t off = static_cast<size_t>(row) * D;
     const float rstd = nrstd;
     float xh[MAXV][8], g[MAXV][8];
-    Raw8<T> res[MAXV];
+    Raw8<T> res[kResAhead ? MAXV : 1];
     float dot = 0.f;
 #pragma unroll
     for (int i = 0; i < MAXV; ++i) {
@@ -242,7 +246,7 @@ rmsnorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* _
         unpack8<T>(nx[i], xh[i]);
         unpack8<T>(ng[i], g[i]);
         unpack8<T>(wv[i], wf);
-        if (dres) res[i] = nr[i];
+        if (kResAhead && dres) res[i] = nr[i];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           xh[i][j] *= rstd;
@@ -264,7 +268,8 @@ rmsnorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* _
         for (int j = 0; j < 8; ++j) o[j] = rstd * (g[i][j] - xh[i][j] * mean_dot);
         if (dres) {
           float r[8];
-          unpack8<T>(res[i], r);
+          if constexpr (kResAhead) unpack8<T>(res[i], r);
+          else load8<T>(dres + off + v * 8, r);
 #pragma unroll
           for (int j = 0; j < 8; ++j) o[j] += r[j];
         }

@@ -100,7 +100,7 @@ def test_linear_autograd(dev):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("rows,D", [(37, 256), (512, 4096), (5, 8192)])
+@pytest.mark.parametrize("rows,D", [(37, 256), (512, 4096), (5, 8192), (700, 3080), (700, 6152)])
 def test_rmsnorm_fwd_bwd(dev, dtype, rows, D):
     from tesseract_b200 import ops
     x = torch.randn(rows, D, device=dev).to(dtype).requires_grad_()
