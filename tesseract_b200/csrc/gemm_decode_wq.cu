@@ -676,16 +676,22 @@ void plan_tiles(int M, int N, int kb, bool fp8, int fixed_bn, int* bn_out, int* 
 // Y [R, N] = X [R, K] W^T for up to four batch rows: the weights stream through registers and CUDA cores. What bounds it is the bytes
 // in flight, and for small matrices the time until the first are there, so nothing is staged: a CTA of 16 warps per SM owns a run of
 // weight rows, `kw` warps share a row's K (256 elements each in turn) and the other warps take other rows; a warp requests its 512
-// bytes of B = 8 rows (4 for several batch rows, whose sums take the registers) at once, and those of its next step before it uses these. The first request is made before the kernel waits for
-// the one before it (weights do not depend on it). The tensor-core kernel above needs a cluster to cut K for matrices of few rows, and
-// pays its barriers and reduction with every launch.
-// Measured on B200, launches behind one another, us here / above, [N, K] = 4096 x 4096, 6144 x 4096, 4096 x 14336, 28672 x 4096,
-// 1024 x 1024: one row 7.9 / 13.3, 10.8 / 14.6, 24.8 / 32.7, 40.1 / 40.5, 2.3 / 6.2; two rows 9.5 / 13.5, 13.8 / 14.4, 30.6 / 33.0,
-// 54 / 40, 2.2 / 6.4; four rows 11.2 / 13.2, 16.3 / 14.5, 36 / 33, 65 / 40, 2.5 / 6.4. So it takes one row of matrices whose rows are
-// too few to fill the SMs with tiles, and several while the multiply-adds of all of them are few.
+// bytes of B = 8 rows (4 for several batch rows, whose sums take the registers) at once, and those of its next step before it uses
+// these. The first request is made before the kernel waits for the one before it (weights do not depend on it). The tensor-core kernel
+// above needs a cluster to cut K for matrices of few rows, and pays its barriers and reduction with every launch.
+// Measured on B200, launches behind one another, us here / above, by [N, K]:
+//   one row    1024 x 1024 2.3 / 6.2   4096 x 4096 8.0 / 13.2   6144 x 4096 10.9 / 14.6   4096 x 14336 25 / 32   8192 x 24576 68 / 104
+//              16384 x 4096 25.2 / 26.5   16384 x 5120 32.9 / 31.8   28672 x 4096 40.1 / 40.5
+//   two rows   4096 x 5120 12.6 / 15.1   6144 x 4096 13.8 / 14.8   5120 x 5120 16.7 / 15.6   7168 x 4352 19.1 / 15.1
+//   four rows  4096 x 4096 11.3 / 13.3   7168 x 2304 12.7 / 13.6   256 x 64 2.3 / 2.1   28672 x 4096 65 / 40
+// So it takes one row unless the matrix has enough rows to fill the SMs with tiles and is large besides, and several rows while the
+// multiply-adds of all of them are few: 2^26, or 3/4 of that where the kernel above has tiles enough without a cluster (N > 4096).
 constexpr int kRowsMaxK = 24576;                       // (rows of X fit shared memory)
 bool rows_kernel_pays(int M, int N, int K) {
-  return K <= kRowsMaxK && (M == 1 ? N <= 16384 : M <= 4 && static_cast<long long>(M) * N * K <= (1ll << 26));
+  const long long weights = static_cast<long long>(N) * K;
+  if (K > kRowsMaxK || M > 4) return false;
+  if (M == 1) return N <= 8192 || (N <= 16384 && weights <= 1ll << 26);
+  return M * weights <= (N <= 4096 ? 4ll << 24 : 3ll << 24) && (M == 2 || K > 64);
 }
 constexpr int kRowsThreads = 512, kRowsWarps = 16, kRowsChunk = 256;
 
@@ -782,9 +788,15 @@ gemv_rows_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __res
 cudaError_t launch_rows(const void* X, const void* W, void* Y, int M, int N, int K, long long ldx, long long ldw, long long ldy, int pdl,
                         cudaStream_t s) {
   const int chunks = (K + kRowsChunk - 1) / kRowsChunk;
-  int kw = kRowsWarps;
-  while (kw > 1 && kw > chunks) kw /= 2;
   const int sms = sm_count(), per = (N + sms - 1) / sms, grid = (N + per - 1) / per;
+  // the warps per row that take the fewest steps: rows of 9 or 17 chunks on 8 or 16 warps leave nearly half of them idle
+  int kw = kRowsWarps;
+  auto steps = [&](int w) {
+    const int rows = kRowsWarps / w * (M == 1 ? 8 : 4);
+    return static_cast<long long>((chunks + w - 1) / w) * ((per + rows - 1) / rows);
+  };
+  for (int w = kRowsWarps / 2; w >= 1; w /= 2)
+    if (steps(w) < steps(kw)) kw = w;
   auto go = [&](auto kern, int rows) {
     const int bytes = rows * K * 2;
     // (the most that any K takes: another thread may be between its own call of this and its launch)

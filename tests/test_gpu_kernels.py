@@ -370,10 +370,11 @@ def test_flash_forward_accuracy_over_score_widths(dev, B, H, Hkv, Sq, Sk, D, wid
 
 
 @pytest.mark.parametrize("M", [1, 2, 3, 4])
-@pytest.mark.parametrize("N,K", [(1, 16), (7, 272), (149, 4096), (2049, 528), (33, 24576), (1000, 1040)])
+@pytest.mark.parametrize("N,K", [(1, 16), (7, 272), (149, 4096), (2049, 528), (33, 24576), (1000, 1040), (2049, 2304), (600, 4352), (5000, 272),
+                                 (28672, 4096)])                              # (the last, and K = 16 with three rows on, by the tensor cores)
 @pytest.mark.parametrize("pdl", [False, True])
 def test_few_rows_gemv(dev, M, N, K, pdl):
-    """One to four rows on CUDA cores: ends of rows, of K and of its share per warp. fp32 sums rounded to bf16 once: 0.0011 of a
+    """One to four rows on CUDA cores: ends of rows, of K and of its share per warp, 1 to 16 warps per row. fp32 sums rounded to bf16 once: 0.0011 of a
     value in the mean. Rows of the result beside the written ones stay as they were."""
     from tesseract_b200.ops.gemm import stream_linear
     g = torch.Generator(device=dev).manual_seed(M * N + K)
