@@ -551,8 +551,13 @@ TSB_EXPORT int tsb_flash_bwd(const void* dO, const void* q, const void* k, const
   p.status = device_status_word();
   auto go = [&](auto dim, auto kern, auto rows_kern, auto dq_kern) -> int {
     constexpr int kD = decltype(dim)::value;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdCfg<kD>::kSmemBytes);
-    if (e != cudaSuccess) return static_cast<int>(e);
+    static PerDeviceFlag attr_set;                      // (one per D)
+    cudaError_t e = cudaSuccess;
+    if (attr_set.unset()) {
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdCfg<kD>::kSmemBytes);
+      if (e != cudaSuccess) return static_cast<int>(e);
+      attr_set.set();
+    }
     rows_kern<<<static_cast<unsigned>((rows * (kD / 8) + 255) / 256), 256, 0, s>>>(
         static_cast<const __nv_bfloat16*>(dO), static_cast<const __nv_bfloat16*>(o), lse, lse2, delta, dq_acc, rows, Sq, n_q * BT, H);
     kern<<<dim3(static_cast<unsigned>(Hkv) * ((Sk + BT - 1) / BT), 1, B), kBwdThreads, BwdCfg<kD>::kSmemBytes, s>>>(tq, tk, tv, tdo, p);

@@ -877,7 +877,8 @@ TSB_EXPORT int tsb_gemm_decode_wq(const void* X, const void* W, const float* w_s
 #undef TSB_WQ_ARGS
 }
 
-// The plan the call above makes for a problem (host only): *bn (pass a positive value to fix the tile width, as for
+// The plan the call above makes for a problem on the tensor cores (host only; where neither width nor split is given, up to four bf16
+// rows may take the kernel for few rows instead, which has neither): *bn (pass a positive value to fix the tile width, as for
 // packed weights), *split, and the ring depth it leads to.
 TSB_EXPORT int tsb_gemm_decode_wq_plan(int M, int N, int K, int w_fp8, int* bn, int* split, int* w_stages,
                                        int* resident) {

@@ -126,7 +126,7 @@ _native.register_signatures({
 
 
 def stream_linear_plan(M: int, N: int, K: int, fp8: bool, bn: int = 0):
-    """(tile width, K split) the streaming kernel chooses on the current device (``bn`` > 0 fixes the width)."""
+    """(tile width, K split) the streaming kernel chooses on the tensor cores of the current device (``bn`` > 0 fixes the width)."""
     import ctypes
     b, s_, st, res = ctypes.c_int(bn), ctypes.c_int(0), ctypes.c_int(0), ctypes.c_int(0)
     _native.check(_native.lib().tsb_gemm_decode_wq_plan(M, N, K, int(fp8), ctypes.byref(b), ctypes.byref(s_),
