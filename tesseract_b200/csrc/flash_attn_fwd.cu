@@ -709,17 +709,19 @@ flash_bounded_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 // O accumulates in TMEM over all key tiles and exponents refer to a row's running maximum, so that the largest probability of a row
 // is 1 and exact in bf16. (With a reference that may stay up to 2^8 behind, O need hardly ever be rescaled, but the largest
 // probability is rounded like the others: error of O before its own rounding with scores three / six times as wide as unit ones 0.0006 /
-// 0.0004 -> 0.0015 / 0.0012.) Where the maximum of any row of a warp has grown, the warp rescales O 16 columns at a time between the
-// exponentials of the first 64 keys, which hide the way to TMEM and back: by itself in front of them 0 - 14 % more with heads of 64.
-// Tiles that are masked sum the rounded probabilities, as few of them may make up a row.
+// 0.0004 -> 0.0015 / 0.0012.) Where the maximum of any row of a warp has grown, the warp rescales O: with heads of 64 16 columns at a
+// time between the exponentials of the first 64 keys, which hide the way to TMEM and back (in front of them: 103 -> 114 us for 4 heads,
+// 8192 tokens); with heads of 128 in a short loop in front of them (between them the code of a tile exists twice more, and what it
+// saves is lost to its size: 14 x 423 tokens, 32 heads 102 against 84 us, 16384 tokens 2.23 against 2.21 ms). Tiles that are masked
+// sum the rounded probabilities, as few of them may make up a row.
 //
-// A pair of tiles takes about 3800 clocks per 128 keys, 2048 of them MMAs: a stage's softmax and its MMAs follow one another and two
+// A pair of tiles takes about 3700 clocks per 128 keys, 2048 of them MMAs: a stage's softmax and its MMAs follow one another and two
 // stages fill TMEM, so every instruction of the softmax is packed (f32x2) or left out. With heads of 64 the exponentials (16 per
 // clock) take twice as long as the MMAs; with heads of 128 leaving them out changes 2 %. Measured against one tile per CTA with P in
-// shared memory and O in registers, which this kernel replaced (32 / 8 heads of 128, causal): 2 x 4096 tokens 563 -> 288 us (950
-// TFLOP/s), 16384 tokens 4.07 -> 1.97 ms (1120 TFLOP/s), 2 x 512 queries over 4608 keys 153 -> 81 us; 16 heads of 64, 4 x 1500 tokens,
-// full: 162 -> 78 us (reference up to 2^8 behind: 262 us, 1.83 ms, 78, 76 us). Every fourth exponential as a polynomial on
-// the FMA units was slower (16384 tokens: 1.80 -> 1.92 ms).
+// shared memory and O in registers, which this kernel replaced (32 / 8 heads of 128, causal): 2 x 4096 tokens 580 -> 286 us (960
+// TFLOP/s), 16384 tokens 4.13 -> 1.99 ms (1110 TFLOP/s), 2 x 512 queries over 4608 keys 151 -> 81 us; 16 heads of 64, 4 x 1500 tokens,
+// full: 162 -> 79 us. (With a reference up to 2^8 behind: 268 us, 1.89 ms, 77, 76 us.) Every fourth exponential as a polynomial on the
+// FMA units was slower (16384 tokens: 1.80 -> 1.92 ms).
 constexpr int kPairThreads = 384;
 // Registers per thread: 168 at the launch, 208 for the softmax warps and 88 for the rest after it (256 x 208 + 128 x 88 = 384 x 168).
 constexpr int kPairSoftmaxRegs = 208, kPairOtherRegs = 88;
@@ -730,6 +732,7 @@ struct PairCfg {
   static constexpr int kSlots = D == 128 ? 4 : 8;                       // ring of K and V tiles
   static constexpr int kSmemBytes = kTileBytes * (2 + kSlots) + 1024;
   static constexpr bool kOwnP = D == 64;                                // P beside the scores, not over them
+  static constexpr bool kRescaleBetween = D == 64;                      // O is rescaled between exponentials, not in front of them
   static constexpr int kTmemCols = 512, kColP = kOwnP ? 256 : 0, kPStride = kOwnP ? 64 : BKV, kColO = kOwnP ? 384 : 256;
 };
 
@@ -741,8 +744,8 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 
 // The two tiles of a CTA: neighbouring tiles of a head, the same tile of two heads, or one tile alone. Alone where all tiles together
 // are at most one per SM: two of them on an SM wait for each other's MMAs and issue slots, and the other SM idles. One / two per CTA in
-// us (one tile per CTA of the kernel before): 8 heads of 128, 128 queries over 8192 keys 119 / 134 (129); 16 heads, 512 over 4608 72 / 80
-// (77); 4 heads, 1000 causal 22 / 27 (23); 32 heads of 64, 256 over 4096 47 / 58 (66). With more tiles than SMs, two per CTA cost less
+// us (one tile per CTA of the kernel before): 8 heads of 128, 128 queries over 8192 keys 121 / 133 (128); 16 heads, 512 over 4608 72 / 80
+// (78); 4 heads, 1000 causal 20 / 24 (23); 32 heads of 64, 256 over 4096 47 / 58 (66). With more tiles than SMs, two per CTA cost less
 // than a second round of CTAs.
 enum class PairOf { kTiles, kHeads, kOne };
 
@@ -969,20 +972,44 @@ flash_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           tc_fence_after();
         }
         const bool fresh = m_ref == -INFINITY;                     // no visible scores of this row yet: O and l hold nothing of it
+        if (fresh) m_ref = m_tile;
         const bool grow = m_tile > m_ref;
-        const float factor = grow && !fresh ? exp2f((m_ref - m_tile) * p.scale_log2) : 1.f;
-        if (grow) m_ref = m_tile;
+        // warp-collective: every lane rescales its own TMEM lane (factor 1 where nothing changed)
+        const bool rescale = __any_sync(0xffffffffu, grow);
+        float factor = 1.f;
+        if (rescale) {
+          if (grow) {
+            factor = exp2f((m_ref - m_tile) * p.scale_log2);
+            m_ref = m_tile;
+          }
+          l2a = mul_f32x2(l2a, both(factor));
+          l2b = mul_f32x2(l2b, both(factor));
+          if constexpr (!Cfg::kRescaleBetween) {
+#pragma unroll 1
+            for (int c = 0; c < D / 32; ++c) {
+              uint32_t r[32];
+              tmem_ld_32x32(o_addr + c * 32, r);
+              tmem_ld_wait();
+#pragma unroll
+              for (int n = 0; n < 32; n += 2) {
+                const float2 o = mul_f32x2(make_float2(__uint_as_float(r[n]), __uint_as_float(r[n + 1])), both(factor));
+                r[n] = __float_as_uint(o.x);
+                r[n + 1] = __float_as_uint(o.y);
+              }
+              tmem_st_32x32(o_addr + c * 32, r);
+            }
+          }
+        }
         const float2 base = both(m_ref == -INFINITY ? 0.f : -m_ref * p.scale_log2);
-        auto probabilities = [&](auto rescale) {
-          constexpr bool kRescale = decltype(rescale)::value;
+        auto probabilities = [&](auto between) {
+          constexpr bool kBetween = decltype(between)::value;
 #pragma unroll
           for (int c = 0; c < BKV / 64; ++c) {
-            uint32_t packed[32];
-            uint32_t r[16];
+            uint32_t packed[32], r[16];
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
               constexpr int kEvery = 32 / (D / 16);                // pairs of exponentials per 16 columns of O
-              if (kRescale && c == 0 && i % kEvery == 0) tmem_ld_32x16(o_addr + i / kEvery * 16, r);
+              if (kBetween && c == 0 && i % kEvery == 0) tmem_ld_32x16(o_addr + i / kEvery * 16, r);
               const int e = c * 64 + 2 * i;
               const float2 t = fma_f32x2(make_float2(__uint_as_float(sr[e]), __uint_as_float(sr[e + 1])), mul, base);
               float2 x = make_float2(exp2_ftz(t.x), exp2_ftz(t.y));
@@ -994,7 +1021,7 @@ flash_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
               if constexpr (kMask) x = make_float2(__uint_as_float(packed[i] << 16), __uint_as_float(packed[i] & 0xffff0000u));
               if (i & 1) l2b = add_f32x2(l2b, x);
               else l2a = add_f32x2(l2a, x);
-              if (kRescale && c == 0 && i % kEvery == kEvery - 1) {
+              if (kBetween && c == 0 && i % kEvery == kEvery - 1) {
                 tmem_ld_wait();
 #pragma unroll
                 for (int n = 0; n < 16; n += 2) {
@@ -1011,11 +1038,9 @@ flash_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
             mbar_arrive(c ? &p_full[s] : &p_half[s]);
           }
         };
-        // warp-collective: every lane rescales its own TMEM lane (factor 1 where nothing changed)
-        if (j > 0 && __any_sync(0xffffffffu, grow && !fresh)) {
-          l2a = mul_f32x2(l2a, both(factor));
-          l2b = mul_f32x2(l2b, both(factor));
-          probabilities(std::true_type{});
+        if constexpr (Cfg::kRescaleBetween) {
+          if (rescale) probabilities(std::true_type{});
+          else probabilities(std::false_type{});
         } else {
           probabilities(std::false_type{});
         }
