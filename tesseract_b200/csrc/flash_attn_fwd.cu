@@ -6,7 +6,7 @@
 // Causal masking follows the reference: key j is visible to query i iff j <= i + (Sk - Sq); a fully masked
 // row produces zeros; softmax statistics are fp32; scale is folded into the exponent
 // (src/cuda/FusedAttention.cu:69-80,318-331,368-567 is the WMMA kernel this replaces).
-// Also writes the per-row log-sum-exp needed by the backward kernel.
+// Of plain scores also the per-row log-sum-exp that the backward kernel needs.
 #include "attn_form.cuh"
 
 #include <algorithm>
@@ -35,7 +35,7 @@ struct FaParams {
   int B, Sq, Sk, H, Hkv;
   long long o_sb, o_ss, o_sh;
   const int* cu_seqlens;  // varlen: int32 [B + 1] row offsets of the sequences in the packed token axis, else null
-  const int* cu_keys;     // varlen: row offsets of the sequences' keys on a key axis of their own, null: the token axis
+  const int* cu_keys;     // varlen: row offsets of the sequences' keys on a key axis of their own, null: the token axis (plain scores only)
   float scale_log2;  // softmax scale * log2(e)
   float scale;
   int causal;
@@ -71,26 +71,14 @@ __device__ __forceinline__ uint64_t mnmajor_desc(uint32_t base, int ks, uint32_t
 template <int D>
 __global__ void __launch_bounds__(kFaThreads, 1)
 flash_form_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                 const __grid_constant__ CUtensorMap tmV, FaParams p_in) {
+                 const __grid_constant__ CUtensorMap tmV, FaParams p) {
   using Cfg = FaCfg<D>;
-  // Variable-length batches: the sequences sit one after another on ONE token axis (tensor maps with batch 1);
-  // block z handles sequence z, whose rows start at cu_seqlens[z]. Tiles that reach past its end read rows of the
-  // next sequence (or the zero fill) and the length mask below discards them.
-  FaParams p = p_in;
-  // With `cu_keys` the keys of a sequence are rows of a second axis and may outnumber the queries: the queries are then
-  // the last Sq of its Sk positions.
-  int row0 = 0, krow0 = 0;
-  int bb = blockIdx.z;
-  if (p_in.cu_seqlens) {
-    row0 = krow0 = p_in.cu_seqlens[blockIdx.z];
-    p.Sq = p.Sk = p_in.cu_seqlens[blockIdx.z + 1] - row0;
-    if (p_in.cu_keys) {
-      krow0 = p_in.cu_keys[blockIdx.z];
-      p.Sk = p_in.cu_keys[blockIdx.z + 1] - krow0;
-    }
-    bb = 0;
-    if (static_cast<int>(gridDim.x - 1 - blockIdx.x) * BQ >= p.Sq) return;  // no query rows: the whole CTA leaves
-  }
+  // The sequences sit one after another on ONE token axis (tensor maps with batch 1), their keys on a second one; block z handles
+  // sequence z, whose rows start at cu_seqlens[z]. Tiles that reach past its end read rows of the next sequence (or the zero fill)
+  // and the length mask below discards them. The queries are the last Sq of Sk positions.
+  const int row0 = p.cu_seqlens[blockIdx.z], krow0 = p.cu_keys[blockIdx.z];
+  const int Sq = p.cu_seqlens[blockIdx.z + 1] - row0, Sk = p.cu_keys[blockIdx.z + 1] - krow0;
+  if (static_cast<int>(gridDim.x - 1 - blockIdx.x) * BQ >= Sq) return;  // no query rows: the whole CTA leaves
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;
@@ -107,17 +95,12 @@ flash_form_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   const int lane = threadIdx.x & 31;
   const int qt = gridDim.x - 1 - blockIdx.x;  // heavy (late) query tiles first under causal masking
   const int h = blockIdx.y;
-  const int b = blockIdx.z;
   const int hk = h / (p.H / p.Hkv);
   const int q0 = qt * BQ;
-  const int offset = p.Sk - p.Sq;
+  const int offset = Sk - Sq;
 
-  int n_tiles = (p.Sk + BKV - 1) / BKV;
-  if (p.causal) {
-    const int last_col = q0 + BQ - 1 + offset;
-    const int lim = last_col < 0 ? 0 : last_col / BKV + 1;
-    n_tiles = min(n_tiles, lim);
-  }
+  const int last_col = q0 + BQ - 1 + offset;
+  int n_tiles = min((Sk + BKV - 1) / BKV, last_col < 0 ? 0 : last_col / BKV + 1);
   int j0 = 0;                  // first key tile
   if (p.form.window > 0) j0 = max(0, q0 + offset - p.form.window + 1) / BKV;
   n_tiles = max(0, n_tiles - j0);
@@ -154,7 +137,7 @@ flash_form_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     if (lane == 0 && n_tiles > 0) {
       mbar_expect_tx(&q_full, Cfg::kTileBytes);
 #pragma unroll
-      for (int hf = 0; hf < Cfg::kHalves; ++hf) tma_load_4d(sQ + hf * 16384, &tmQ, &q_full, hf * 64, q0 + row0, h, bb);
+      for (int hf = 0; hf < Cfg::kHalves; ++hf) tma_load_4d(sQ + hf * 16384, &tmQ, &q_full, hf * 64, q0 + row0, h, 0);
       for (int j = 0; j < n_tiles; ++j) {
         const int st = j & 1;
         const uint32_t par = ((j >> 1) & 1) ^ 1u;
@@ -162,12 +145,12 @@ flash_form_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         mbar_expect_tx(&k_full[st], Cfg::kTileBytes);
 #pragma unroll
         for (int hf = 0; hf < Cfg::kHalves; ++hf)
-          tma_load_4d(sK + st * Cfg::kTileBytes + hf * 16384, &tmK, &k_full[st], hf * 64, (j0 + j) * BKV + krow0, hk, bb);
+          tma_load_4d(sK + st * Cfg::kTileBytes + hf * 16384, &tmK, &k_full[st], hf * 64, (j0 + j) * BKV + krow0, hk, 0);
         if (!mbar_wait(&v_empty[st], par, &cta_abort, p.status)) break;
         mbar_expect_tx(&v_full[st], Cfg::kTileBytes);
 #pragma unroll
         for (int hf = 0; hf < Cfg::kHalves; ++hf)
-          tma_load_4d(sV + st * Cfg::kTileBytes + hf * 16384, &tmV, &v_full[st], hf * 64, (j0 + j) * BKV + krow0, hk, bb);
+          tma_load_4d(sV + st * Cfg::kTileBytes + hf * 16384, &tmV, &v_full[st], hf * 64, (j0 + j) * BKV + krow0, hk, 0);
       }
     }
   } else if (warp == 5) {
@@ -233,19 +216,14 @@ flash_form_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       tc_fence_after();
       const uint32_t s_addr = tmem_base + lane_addr + (st ? Cfg::kColS1 : Cfg::kColS0);
       const int c0 = (j0 + j) * BKV;
-      const bool need_mask = raw && ((p.causal && c0 + BKV - 1 > q0 + offset) || (c0 + BKV > p.Sk) ||
-                                     (p.form.window > 0 && c0 < q0 + BQ + offset - p.form.window));
+      const bool need_mask = raw && (c0 + BKV - 1 > q0 + offset || c0 + BKV > Sk || (p.form.window > 0 && c0 < q0 + BQ + offset - p.form.window));
       const int lo = p.form.window > 0 ? row_limit - p.form.window + 1 - c0 : 0;      // first visible column
       int vis = BKV;  // number of visible columns of this tile for this row
-      if (need_mask) {
-        int lim = p.Sk - c0;
-        if (p.causal) lim = min(lim, row_limit - c0 + 1);
-        vis = max(0, min(BKV, lim));
-      }
+      if (need_mask) vis = max(0, min(BKV, min(Sk - c0, row_limit - c0 + 1)));
       // pass 1: row maximum (tiles that need no masking skip the per-element visibility test)
       float m_tile = -INFINITY;
       if (!raw) {
-        const int hi = min(p.Sk - 1, row_limit) - c0;                                    // visible columns: lo .. hi
+        const int hi = min(Sk - 1, row_limit) - c0;                                      // visible columns: lo .. hi
 #pragma unroll 1
         for (int c = 0; c < BKV / 32; ++c) {
           uint32_t r[32];
@@ -372,7 +350,7 @@ flash_form_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         ok = false;
       }
     }
-    if (ok && qi < p.Sq) {
+    if (ok && qi < Sq) {
       float inv_l = l_run > 0.f ? 1.f / l_run : 0.f;
       if (p.form.sink && l_run > 0.f) inv_l = 1.f / (l_run + exp2f(p.form.sink[h] * kLog2e - m_run * mul));
       if (p.gate.kind != 2) inv_l *= p.gate.factor<__nv_bfloat16>(row0 + qi, h, D, 0);
@@ -390,7 +368,7 @@ flash_form_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           }
         }
       }
-      __nv_bfloat16* orow = p.o + bb * p.o_sb + static_cast<long long>(row0 + qi) * p.o_ss + h * p.o_sh;
+      __nv_bfloat16* orow = p.o + static_cast<long long>(row0 + qi) * p.o_ss + h * p.o_sh;
 #pragma unroll
       for (int c = 0; c < D / 8; ++c) {
         uint4 v;
@@ -399,10 +377,6 @@ flash_form_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         v.z = pack_bf16x2(o_acc[c * 8 + 4] * inv_l, o_acc[c * 8 + 5] * inv_l);
         v.w = pack_bf16x2(o_acc[c * 8 + 6] * inv_l, o_acc[c * 8 + 7] * inv_l);
         *reinterpret_cast<uint4*>(orow + c * 8) = v;
-      }
-      if (p.lse) {
-        const float lse = l_run > 0.f ? (m_run * p.scale + __logf(l_run)) : -INFINITY;
-        p.lse[(static_cast<long long>(b) * p.H + h) * p.Sq + qi] = lse;
       }
     }
   }
@@ -744,8 +718,8 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 
 // The two tiles of a CTA: neighbouring tiles of a head, the same tile of two heads, or one tile alone. Alone where all tiles together
 // are at most one per SM: two of them on an SM wait for each other's MMAs and issue slots, and the other SM idles. One / two per CTA in
-// us (one tile per CTA of the kernel before): 8 heads of 128, 128 queries over 8192 keys 121 / 133 (128); 16 heads, 512 over 4608 72 / 80
-// (78); 4 heads, 1000 causal 20 / 24 (23); 32 heads of 64, 256 over 4096 47 / 58 (66). With more tiles than SMs, two per CTA cost less
+// us (one tile per CTA of the kernel before): 8 heads of 128, 128 queries over 8192 keys 121 / 133 (129); 16 heads, 512 over 4608 72 / 80
+// (77); 4 heads, 1000 causal 21 / 25 (23); 32 heads of 64, 256 over 4096 47 / 58 (66). With more tiles than SMs, two per CTA cost less
 // than a second round of CTAs.
 enum class PairOf { kTiles, kHeads, kOne };
 
