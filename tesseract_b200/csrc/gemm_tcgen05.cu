@@ -723,9 +723,10 @@ TSB_EXPORT int tsb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
     auto tiles = [&](int b) { return mt * ((N + b - 1) / b); };
     // 128 x 256 tiles would be chosen, and tiles of 256 x 256 for pairs of SMs take no more rounds than they. Time of the former over that of
     // the latter, sustained: K = 256 0.82, 512 0.98, 768 0.96 - 1.01, 896 0.97 - 1.07, 960 1.08, 1024 - 1536 1.00 - 1.14 (9001 x 1288 x 1000
-    // 1.21), 2048 - 8192 1.00 - 1.08 (two rounds of which the second is a third full 1.00, 8192 x 28672 x 4096 1.05), 9216 - 12288 1.00 - 1.02,
-    // beyond 0.975 - 1.01 (4096 x 4096 x 128256 0.975, 8192 x 4096 x 28672 0.985, 17408 1.007). (Runs of one side differ by 1 %.)
-    if (max_ctas <= 0 && N >= 256 && tiles(256) >= sms && K >= 960 && K <= 12288) {
+    // 1.21), 2048 - 8192 1.00 - 1.08 (two rounds of which the second is a third full 1.00, 8192 x 28672 x 4096 1.05), 9216 - 12288 1.00 - 1.02.
+    // Beyond, 1.00 - 1.06 where the rows of both operands run along M and N (weight gradients: 4096 x 4096 x 16384 1.04), else 0.975 - 1.01
+    // (4096 x 4096 x 128256 0.975, 4096 x 4096 x 32768 0.98, 17408 1.007). (Runs of one side differ by 1 %.)
+    if (max_ctas <= 0 && N >= 256 && tiles(256) >= sms && K >= 960 && (K <= 12288 || (a_mn && b_mn))) {
       const long long pairs = sms / 2, tiles2 = ((M + 255) / 256) * static_cast<long long>((N + 255) / 256);
       pair = (tiles2 + pairs - 1) / pairs <= (tiles(256) + sms - 1) / sms;
     }

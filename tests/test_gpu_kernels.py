@@ -473,7 +473,8 @@ def test_tiny_llama_train_step_matches_cpu(dev):
 
 
 @pytest.mark.parametrize("M,N,K,pad", [(4864, 4096, 64, 0), (4872, 4104, 520, 0), (9000, 2312, 136, 0),      # 128 x 256 tiles; from here on pairs
-                                       (4864, 4096, 960, 0), (4872, 4104, 1032, 0), (9000, 2312, 1000, 3), (4864, 4096, 12288, 0)])
+                                       (4864, 4096, 960, 0), (4872, 4104, 1032, 0), (9000, 2312, 1000, 3), (4864, 4096, 12288, 0),
+                                       (4864, 4096, 12352, 0)])                                  # the last: pairs for both operands along M and N
 @pytest.mark.parametrize("a_mn", [False, True])
 @pytest.mark.parametrize("b_mn", [False, True])
 @pytest.mark.parametrize("out,accumulate", [(torch.bfloat16, False), (torch.bfloat16, True), (torch.float32, True)])
