@@ -27,8 +27,8 @@
 //
 // Measured, all of the backward pass (32 / 8 heads of 128, causal): 2 x 4096 tokens 1.89 -> 0.85 ms, 16384 tokens 13.6 -> 6.2 ms
 // (890 TFLOP/s) against four warps that went through scores, P, dS and dQ of a tile one after another; 16 heads of 64,
-// 4 x 1500 tokens, full: 400 -> 250 us. What bounds it now: the atomics of dQ for heads of 128 (below), else the chain from
-// scores over P and dS to the products (about 4200 clocks a step, of which the tensor core works 2560).
+// 4 x 1500 tokens, full: 382 -> 210 us. What bounds it now: the atomics of dQ for heads of 128 (above), for heads of 64 the chain from
+// scores over P and dS to the products (about 4200 clocks a step, of which the tensor core works 1280).
 //
 // A kernel before it writes delta_i = rowsum(dO_i * O_i) and lse_i in units of log 2 (+inf where a row sees no key or does not
 // exist: P is 0 there) and zeroes the scratch; one after it turns dQ into bf16.
