@@ -36,8 +36,7 @@ struct TileCoord {
   int m_blk, n_blk;
 };
 
-template <int GM = 16>
-__device__ __forceinline__ TileCoord tile_coord(int t, int num_m, int num_n) {
+__device__ __forceinline__ TileCoord tile_coord(int t, int num_m, int num_n, int GM = 16) {
   const int group_size = GM * num_n;
   const int group_id = t / group_size;
   const int first_m = group_id * GM;
@@ -173,7 +172,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   __shared__ uint32_t tmem_base_smem;
   __shared__ volatile int cta_abort;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
 
   const int num_m = (M + BM - 1) / BM;
@@ -212,31 +211,33 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
-        const TileCoord tc = (gmode == 2) ? tile_coord(t % tiles_per_group, num_m, num_n) : tile_coord(t / split_k, num_m, num_n);
-        const int m0 = tc.m_blk * BM;
-        const int n0 = tc.n_blk * BN;
-        int kb0 = (t % split_k) * kb_per;
-        int kb1 = min(total_kb, kb0 + kb_per);
-        int b_row_off = 0;  // rows of the stacked B tensor map before this tile's group
-        const int a_row = m0 + input_row_offset(grp, n0);
-        if (gmode == 1) {
-          if (m0 >= m_limit) continue;
-          b_row_off = static_cast<int>(group_of_row(grp, m0) * grp.b_group_rows);
-        } else if (gmode == 2) {
-          const int g = t / tiles_per_group;
-          kb0 = __ldg(grp.offsets + g) / BK;
-          kb1 = __ldg(grp.offsets + g + 1) / BK;
-        }
-        bool ok = true;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          ok = mbar_wait(&empty_bar[stage], phase ^ 1u, &cta_abort, status);
-          if (!ok) break;
-          uint8_t* sA = smem + stage * Cfg::kStageBytes;
-          uint8_t* sB = sA + Cfg::kStageBytesA;
+    // (The loops of warps 0 and 1 are walked by the whole warp, and one thread issues: see elect_one.)
+    const bool lead = elect_one();
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
+      const TileCoord tc = (gmode == 2) ? tile_coord(t % tiles_per_group, num_m, num_n) : tile_coord(t / split_k, num_m, num_n);
+      const int m0 = tc.m_blk * BM;
+      const int n0 = tc.n_blk * BN;
+      int kb0 = (t % split_k) * kb_per;
+      int kb1 = min(total_kb, kb0 + kb_per);
+      int b_row_off = 0;  // rows of the stacked B tensor map before this tile's group
+      const int a_row = m0 + input_row_offset(grp, n0);
+      if (gmode == 1) {
+        if (m0 >= m_limit) continue;
+        b_row_off = static_cast<int>(group_of_row(grp, m0) * grp.b_group_rows);
+      } else if (gmode == 2) {
+        const int g = t / tiles_per_group;
+        kb0 = __ldg(grp.offsets + g) / BK;
+        kb1 = __ldg(grp.offsets + g + 1) / BK;
+      }
+      bool ok = true;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        ok = mbar_wait_warp(&empty_bar[stage], phase ^ 1u, &cta_abort, status);
+        if (!ok) break;
+        uint8_t* sA = smem + stage * Cfg::kStageBytes;
+        uint8_t* sB = sA + Cfg::kStageBytesA;
+        if (lead) {
           mbar_expect_tx(&full_bar[stage], Cfg::kStageBytes);
           if (!A_MN) {
             tma_load_2d(sA, &tmA, &full_bar[stage], kb * BK, a_row);
@@ -251,61 +252,61 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             for (int i = 0; i < BN / 64; ++i)
               tma_load_2d(sB + i * 8192, &tmB, &full_bar[stage], n0 + i * 64, kb * BK + b_row_off);
           }
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
         }
-        if (!ok) break;
+        __syncwarp();
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1u;
+        }
       }
+      if (!ok) break;
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc(BM, BN, 1, 1, A_MN ? 1 : 0, B_MN ? 1 : 0);
-      int stage = 0;
-      uint32_t phase = 0;
-      int acc = 0;
-      uint32_t acc_phase = 0;
-      for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
-        int kb0 = (t % split_k) * kb_per;
-        int kb1 = min(total_kb, kb0 + kb_per);
-        if (gmode == 1) {
-          if (tile_coord(t, num_m, num_n).m_blk * BM >= m_limit) continue;
-        } else if (gmode == 2) {
-          const int g = t / tiles_per_group;
-          kb0 = __ldg(grp.offsets + g) / BK;
-          kb1 = __ldg(grp.offsets + g + 1) / BK;
-        }
-        bool ok = mbar_wait(&tmem_empty_bar[acc], acc_phase ^ 1u, &cta_abort, status);
+    const uint32_t lead = elect_one() ? 1u : 0u;
+    constexpr uint32_t idesc = umma_idesc(BM, BN, 1, 1, A_MN ? 1 : 0, B_MN ? 1 : 0);
+    int stage = 0;
+    uint32_t phase = 0;
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
+      int kb0 = (t % split_k) * kb_per;
+      int kb1 = min(total_kb, kb0 + kb_per);
+      if (gmode == 1) {
+        if (tile_coord(t, num_m, num_n).m_blk * BM >= m_limit) continue;
+      } else if (gmode == 2) {
+        const int g = t / tiles_per_group;
+        kb0 = __ldg(grp.offsets + g) / BK;
+        kb1 = __ldg(grp.offsets + g + 1) / BK;
+      }
+      bool ok = mbar_wait_warp(&tmem_empty_bar[acc], acc_phase ^ 1u, &cta_abort, status);
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        ok = mbar_wait_warp(&full_bar[stage], phase, &cta_abort, status);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
-        for (int kb = kb0; kb < kb1; ++kb) {
-          ok = mbar_wait(&full_bar[stage], phase, &cta_abort, status);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t a_base = smem_u32(smem + stage * Cfg::kStageBytes);
-          const uint32_t b_base = a_base + Cfg::kStageBytesA;
+        const uint32_t a_base = smem_u32(smem + stage * Cfg::kStageBytes);
+        const uint32_t b_base = a_base + Cfg::kStageBytesA;
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t adesc = A_MN ? umma_smem_desc_sw128(a_base + k * 2048, 8192, 1024)
-                                        : umma_smem_desc_sw128(a_base + k * 32, 16, 1024);
-            const uint64_t bdesc = B_MN ? umma_smem_desc_sw128(b_base + k * 2048, 8192, 1024)
-                                        : umma_smem_desc_sw128(b_base + k * 32, 16, 1024);
-            umma_f16(d_tmem, adesc, bdesc, idesc, (kb > kb0 || k != 0) ? 1u : 0u);
-          }
-          umma_commit(&empty_bar[stage]);  // frees the smem stage once these MMAs have read it
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
+        for (int k = 0; k < BK / 16; ++k) {
+          const uint64_t adesc = A_MN ? umma_smem_desc_sw128(a_base + k * 2048, 8192, 1024)
+                                      : umma_smem_desc_sw128(a_base + k * 32, 16, 1024);
+          const uint64_t bdesc = B_MN ? umma_smem_desc_sw128(b_base + k * 2048, 8192, 1024)
+                                      : umma_smem_desc_sw128(b_base + k * 32, 16, 1024);
+          umma_f16_if(lead, d_tmem, adesc, bdesc, idesc, (kb > kb0 || k != 0) ? 1u : 0u);
         }
-        if (!ok) break;
-        umma_commit(&tmem_full_bar[acc]);  // accumulator complete
-        acc ^= 1;
-        if (acc == 0) acc_phase ^= 1u;
+        umma_commit_if(lead, &empty_bar[stage]);  // frees the smem stage once these MMAs have read it
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1u;
+        }
       }
+      if (!ok) break;
+      umma_commit_if(lead, &tmem_full_bar[acc]);  // accumulator complete
+      acc ^= 1;
+      if (acc == 0) acc_phase ^= 1u;
     }
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..5)
@@ -388,16 +389,56 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 }
 
 // ---------------------------------------------------------------- two SMs on one tile
-// The same product on tiles of 256 x 256 that a cluster of two CTAs works on together: `tcgen05.mma.cta_group::2`, issued by the first
-// CTA, multiplies the 256 rows of A (128 in each CTA's shared memory) with the 256 columns of B (128 in each), and each CTA's TMEM
-// receives its 128 rows. Against 128 x 256 tiles per CTA a CTA stages and reads a third less per product (32 instead of 48 KB per
-// 64 of K), so the ring holds six stages instead of four and, which counts under the power limit, fewer bytes move. What it gives depends
-// on K (tsb_gemm_bf16): below, the stores of a tile, which two SMs start together, take longer than its products.
+// The same product on tiles that a cluster of two CTAs works on together: `tcgen05.mma.cta_group::2`, issued by the first CTA, multiplies
+// 256 rows of A (128 in each CTA's shared memory) with n <= 256 columns of B (n / 2 in each), and each CTA's TMEM receives its 128 rows.
+// TMEM holds two such accumulators, and they are used in either of two ways:
+//   whole tiles   256 x 2 n: each block of A that is staged meets two blocks of B, so that 48 KB come in for what two tiles would need 64 KB
+//                 for, and the second product finds A in the tensor core's buffer. What bounds a large product is power, and
+//                 bytes moved through the L2 and shared memory cost it. No accumulator is left to work on during the stores; instead the halves of a tile run
+//                 apart by as many blocks of K as the ring holds, at its end (the first is stored while the second catches up) and at its start.
+//   halves        256 x n, one accumulator after the other: the rest of the tiles where that is at most a round of halves, and products
+//                 that have few tiles or little depth.
+// Rows leave through shared memory and TMA; an accumulated product reads what it adds to while its products are formed.
 //   every CTA   warp 0 loads its halves of A and B; the bytes are counted on the first CTA's barrier. Warps 2-5 store its rows.
 //   first CTA   warp 1 issues the MMAs; its commits arrive in both CTAs.
+// Sustained under the power limit, against tiles of 256 x 256 only, issued by one lane's loop and stored from registers, in turn (us):
+//   forward          8192 x 28672 x 4096 1489 -> 1361    8192 x 4096 x 14336 790 -> 674     3003 x 2048 x 8192 106 -> 86
+//   input gradient   8192 x 4096 x 28672 1575 -> 1362    8192 x 14336 x 4096 796 -> 711     3003 x 2048 x 16384 208 -> 171
+//   weight gradient  28672 x 4096 x 8192 1690 -> 1517    128256 x 4096 x 4096 3788 -> 3502  16384 x 2048 x 3003 179 -> 162
+// (1250 - 1430 TFLOP/s for the large ones.)
 struct PairTile {
-  static constexpr int BM2 = 256, BN2 = 256, kHalfBytes = 128 * BK * 2, kStageBytes = 2 * kHalfBytes, kStages = 6;
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024, kTmemCols = 512;
+  static constexpr int kHalfBytes = 128 * BK * 2;                   // 128 x 64 of an operand
+  static constexpr int kRingBytes = 12 * kHalfBytes;                // four stages of A and two of B, or six of A and one of B
+  static constexpr int kOutBytes = 32 * 128, kOutBufs = 2;          // a storing warp's pieces of C: 32 rows of 128 bytes
+  static constexpr int kSmemBytes = kRingBytes + 4 * kOutBufs * kOutBytes + 1024, kTmemCols = 512;
+};
+
+// How C is cut: `num_m` x `num_w` tiles of 256 rows and `per` times `n` columns. Items below `full` are whole tiles, each two after them
+// the halves of one.
+struct PairPlan {
+  int n, per, group, num_m, num_w, full, items;
+};
+struct PairItem {
+  int m0, c0, halves;
+};
+__device__ __forceinline__ PairItem pair_item(const PairPlan& pl, int t, int N) {
+  const int rest = t - pl.full, tile = rest < 0 ? t : pl.full + (rest >> 1);
+  const TileCoord tc = tile_coord(tile, pl.num_m, pl.num_w, pl.group);
+  const int c0 = (tc.n_blk * pl.per + (rest < 0 ? 0 : rest & 1)) * pl.n;
+  const int fit = c0 >= N ? 0 : c0 + pl.n < N ? 2 : 1;
+  return {tc.m_blk * 256, c0, min(fit, rest < 0 ? pl.per : 1)};
+}
+
+struct RingCursor {
+  int stages, stage = 0;
+  uint32_t phase = 0;
+  __device__ __forceinline__ explicit RingCursor(int n) : stages(n) {}
+  __device__ __forceinline__ void next() {
+    if (++stage == stages) {
+      stage = 0;
+      phase ^= 1u;
+    }
+  }
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -424,43 +465,65 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorM
       ::"r"(smem_u32(smem_dst)), "l"(tmap), "r"(bar), "r"(x), "r"(y)
       : "memory");
 }
-__device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void umma_f16_pair_if(uint32_t pred, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+                                                 uint32_t accumulate) {
   asm volatile(
       "{\n"
-      ".reg .pred p;\n"
+      ".reg .pred p, q;\n"
       "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+      "setp.ne.b32 q, %5, 0;\n"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
       "}\n" ::"r"(tmem_d),
-      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(pred)
+      : "memory");
+}
+// Two products of the same rows of A, one right behind the other: the first leaves them in the tensor core's buffer, the second takes them
+// from there.
+__device__ __forceinline__ void umma_f16_pair_twice_if(uint32_t pred, uint32_t tmem_d0, uint32_t tmem_d1, uint64_t desc_a, uint64_t desc_b0,
+                                                       uint64_t desc_b1, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "setp.ne.b32 p, %6, 0;\n"
+      "setp.ne.b32 q, %7, 0;\n"
+      "@q tcgen05.mma.cta_group::2.kind::f16.collector::a::fill [%0], %2, %3, %5, p;\n"
+      "@q tcgen05.mma.cta_group::2.kind::f16.collector::a::lastuse [%1], %2, %4, %5, p;\n"
+      "}\n" ::"r"(tmem_d0),
+      "r"(tmem_d1), "l"(desc_a), "l"(desc_b0), "l"(desc_b1), "r"(idesc), "r"(accumulate), "r"(pred)
       : "memory");
 }
 // Arrives on the barrier at this offset in both CTAs.
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
-               "h"(static_cast<uint16_t>(3))
-               : "memory");
+__device__ __forceinline__ void umma_commit_pair_if(uint32_t pred, uint64_t* bar) {
+  asm volatile(
+      "{\n"
+      ".reg .pred q;\n"
+      "setp.ne.b32 q, %2, 0;\n"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
+      "}\n" ::"r"(smem_u32(bar)),
+      "h"(static_cast<uint16_t>(3)), "r"(pred)
+      : "memory");
 }
 
 template <bool A_MN, bool B_MN, typename OutT, bool ACCUM>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
-gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, OutT* __restrict__ C, int M, int N, int K,
-                 long long ldc, int* status) {
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
+                 OutT* __restrict__ C, int M, int N, int K, long long ldc, PairPlan pl, int by_tma, int* status) {
   using Cfg = PairTile;
-  constexpr int STAGES = Cfg::kStages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], tmem_full_bar[2], tmem_empty_bar[2];
+  __shared__ __align__(8) uint64_t full_bar[6], empty_bar[6], tmem_full_bar[2], tmem_empty_bar[2];
   __shared__ uint32_t tmem_base_smem;
   __shared__ volatile int cta_abort;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int rank = static_cast<int>(cluster_rank());
-  const int num_m = (M + Cfg::BM2 - 1) / Cfg::BM2, num_n = (N + Cfg::BN2 - 1) / Cfg::BN2, num_tiles = num_m * num_n;
   const int total_kb = (K + BK - 1) / BK;
+  const int stages = pl.per == 2 ? 4 : 6, stage_bytes = (1 + pl.per) * Cfg::kHalfBytes;
+  const int skew = min(stages, total_kb / 2);    // blocks of K by which the halves of a tile start, and end, apart
   const int first = blockIdx.x >> 1, step = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
     cta_abort = 0;
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < 6; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
@@ -471,6 +534,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     mbar_fence_init();
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
+    if (by_tma) tma_prefetch_desc(&tmC);
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_smem)), "r"(Cfg::kTmemCols)
@@ -485,100 +549,202 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int t = first; ok && t < num_tiles; t += step) {
-        const TileCoord tc = tile_coord<8>(t, num_m, num_n);
-        const int m0 = tc.m_blk * Cfg::BM2 + rank * 128, n0 = tc.n_blk * Cfg::BN2 + rank * 128;
-        for (int kb = 0; kb < total_kb; ++kb) {
-          ok = mbar_wait(&empty_bar[stage], phase ^ 1u, &cta_abort, status);
-          if (!ok) break;
-          uint8_t* sA = smem + stage * Cfg::kStageBytes;
-          uint8_t* sB = sA + Cfg::kHalfBytes;
-          if (rank == 0) mbar_expect_tx(&full_bar[stage], 2 * Cfg::kStageBytes);
-          const uint32_t bar = in_first_cta(&full_bar[stage]);
+    // (The whole warp walks the loops of warps 0 and 1 and one thread issues: what a loop computes is then the same for all lanes, as the
+    // copies and MMAs want it.)
+    const bool lead = elect_one();
+    RingCursor at(stages);
+    const int b_half = pl.n / 2;
+    const uint32_t b_bytes = B_MN ? (b_half + 63) / 64 * 8192 : b_half * 128;
+    bool ok = true;
+    for (int t = first; ok && t < pl.items; t += step) {
+      const PairItem it = pair_item(pl, t, N);
+      const int m0 = it.m0 + rank * 128, n0 = it.c0 + rank * b_half;
+      for (int kb = 0; it.halves > 0 && kb < total_kb; ++kb) {
+        ok = mbar_wait_warp(&empty_bar[at.stage], at.phase ^ 1u, &cta_abort, status);
+        if (!ok) break;
+        uint8_t* sA = smem + at.stage * stage_bytes;
+        if (lead) {
+          if (rank == 0) mbar_expect_tx(&full_bar[at.stage], 2 * (Cfg::kHalfBytes + it.halves * b_bytes));
+          const uint32_t bar = in_first_cta(&full_bar[at.stage]);
           if (!A_MN) {
             tma_load_2d_pair(sA, &tmA, bar, kb * BK, m0);
           } else {
 #pragma unroll
             for (int i = 0; i < 2; ++i) tma_load_2d_pair(sA + i * 8192, &tmA, bar, m0 + i * 64, kb * BK);
           }
-          if (!B_MN) {
-            tma_load_2d_pair(sB, &tmB, bar, kb * BK, n0);
-          } else {
-#pragma unroll
-            for (int i = 0; i < 2; ++i) tma_load_2d_pair(sB + i * 8192, &tmB, bar, n0 + i * 64, kb * BK);
-          }
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1u;
+          for (int half = 0; half < it.halves; ++half) {
+            uint8_t* sB = sA + (1 + half) * Cfg::kHalfBytes;
+            if (!B_MN) {
+              tma_load_2d_pair(sB, &tmB, bar, kb * BK, n0 + half * pl.n);
+            } else {
+              for (int i = 0; i < b_half; i += 64) tma_load_2d_pair(sB + i * 128, &tmB, bar, n0 + half * pl.n + i, kb * BK);
+            }
           }
         }
+        __syncwarp();
+        at.next();
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0 && rank == 0) {
-      constexpr uint32_t idesc = umma_idesc(Cfg::BM2, Cfg::BN2, 1, 1, A_MN ? 1 : 0, B_MN ? 1 : 0);
-      int stage = 0, acc = 0;
-      uint32_t phase = 0, acc_phase = 0;
+    if (rank == 0) {
+      const uint32_t lead = elect_one() ? 1u : 0u;
+      const uint32_t idesc = umma_idesc(256, pl.n, 1, 1, A_MN ? 1 : 0, B_MN ? 1 : 0), base = smem_u32(smem);
+      RingCursor at(stages);
+      uint32_t acc = 0, uses = 0;                // the accumulator of the next half, and how often both have been used
       bool ok = true;
-      for (int t = first; ok && t < num_tiles; t += step) {
-        ok = mbar_wait(&tmem_empty_bar[acc], acc_phase ^ 1u, &cta_abort, status);
-        if (!ok) break;
+      auto wait = [&](uint64_t* bar, uint32_t phase) {
+        ok = mbar_wait_warp(bar, phase, &cta_abort, status);
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * Cfg::BN2);
-        for (int kb = 0; kb < total_kb; ++kb) {
-          ok = mbar_wait(&full_bar[stage], phase, &cta_abort, status);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t a_base = smem_u32(smem + stage * Cfg::kStageBytes), b_base = a_base + Cfg::kHalfBytes;
+        return ok;
+      };
+      auto adesc = [&](uint32_t a, int k) { return A_MN ? umma_smem_desc_sw128(a + k * 2048, 8192, 1024) : umma_smem_desc_sw128(a + k * 32, 16, 1024); };
+      auto bdesc = [&](uint32_t b, int k) { return B_MN ? umma_smem_desc_sw128(b + k * 2048, 8192, 1024) : umma_smem_desc_sw128(b + k * 32, 16, 1024); };
+      for (int t = first; ok && t < pl.items; t += step) {
+        const PairItem it = pair_item(pl, t, N);
+        if (it.halves == 0) continue;
+        const uint32_t d0 = tmem_base + acc * 256, d1 = tmem_base + (acc ^ 1) * 256;
+        auto one = [&](int stage, int half, int kb) {
+          const uint32_t a = base + stage * stage_bytes, b = a + (1 + half) * Cfg::kHalfBytes;
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t adesc = A_MN ? umma_smem_desc_sw128(a_base + k * 2048, 8192, 1024) : umma_smem_desc_sw128(a_base + k * 32, 16, 1024);
-            const uint64_t bdesc = B_MN ? umma_smem_desc_sw128(b_base + k * 2048, 8192, 1024) : umma_smem_desc_sw128(b_base + k * 32, 16, 1024);
-            umma_f16_pair(d_tmem, adesc, bdesc, idesc, (kb | k) != 0 ? 1u : 0u);
+          for (int k = 0; k < BK / 16; ++k) umma_f16_pair_if(lead, half ? d1 : d0, adesc(a, k), bdesc(b, k), idesc, (kb | k) != 0 ? 1u : 0u);
+        };
+        if (!wait(&tmem_empty_bar[acc], (uses & 1) ^ 1u)) break;
+        if (it.halves == 1) {
+          for (int kb = 0; kb < total_kb; ++kb) {
+            if (!wait(&full_bar[at.stage], at.phase)) break;
+            one(at.stage, 0, kb);
+            umma_commit_pair_if(lead, &empty_bar[at.stage]);
+            at.next();
           }
-          umma_commit_pair(&empty_bar[stage]);
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1u;
+          if (!ok) break;
+          umma_commit_pair_if(lead, &tmem_full_bar[acc]);
+          uses += acc;
+          acc ^= 1;
+        } else {
+          // `skew` blocks of the first half, then the same blocks of the second
+          RingCursor behind = at;
+          for (int kb = 0; kb < skew; ++kb, at.next()) {
+            if (!wait(&full_bar[at.stage], at.phase)) break;
+            one(at.stage, 0, kb);
           }
+          if (!ok || !wait(&tmem_empty_bar[acc ^ 1], ((uses + acc) & 1) ^ 1u)) break;
+          for (int kb = 0; kb < skew; ++kb, behind.next()) {
+            one(behind.stage, 1, kb);
+            umma_commit_pair_if(lead, &empty_bar[behind.stage]);
+          }
+          for (int kb = skew; kb < total_kb - skew; ++kb, at.next()) {
+            if (!wait(&full_bar[at.stage], at.phase)) break;
+            const uint32_t a = base + at.stage * stage_bytes, b0 = a + Cfg::kHalfBytes, b1 = b0 + Cfg::kHalfBytes;
+#pragma unroll
+            for (int k = 0; k < BK / 16; ++k)
+              umma_f16_pair_twice_if(lead, d0, d1, adesc(a, k), bdesc(b0, k), bdesc(b1, k), idesc, (kb | k) != 0 ? 1u : 0u);
+            umma_commit_pair_if(lead, &empty_bar[at.stage]);
+          }
+          if (!ok) break;
+          behind = at;
+          for (int kb = total_kb - skew; kb < total_kb; ++kb, at.next()) {
+            if (!wait(&full_bar[at.stage], at.phase)) break;
+            one(at.stage, 0, kb);
+          }
+          if (!ok) break;
+          umma_commit_pair_if(lead, &tmem_full_bar[acc]);
+          for (int kb = total_kb - skew; kb < total_kb; ++kb, behind.next()) {
+            one(behind.stage, 1, kb);
+            umma_commit_pair_if(lead, &empty_bar[behind.stage]);
+          }
+          umma_commit_pair_if(lead, &tmem_full_bar[acc ^ 1]);
+          uses += 1;
         }
-        if (!ok) break;
-        umma_commit_pair(&tmem_full_bar[acc]);
-        acc ^= 1;
-        if (acc == 0) acc_phase ^= 1u;
       }
     }
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..5)
     const int q = warp & 3;  // TMEM lane quadrant this warp may read
+    constexpr int kCols = 128 / sizeof(OutT);
     const bool vec_ok = (ldc % (16 / sizeof(OutT)) == 0) && ((reinterpret_cast<uintptr_t>(C) & 15) == 0);
-    int acc = 0;
-    uint32_t acc_phase = 0;
-    for (int t = first; t < num_tiles; t += step) {
-      const TileCoord tc = tile_coord<8>(t, num_m, num_n);
-      const int row = tc.m_blk * Cfg::BM2 + rank * 128 + q * 32 + lane, n0 = tc.n_blk * Cfg::BN2;
-      if (!__all_sync(0xffffffffu, mbar_wait(&tmem_full_bar[acc], acc_phase, &cta_abort, status) ? 1 : 0)) break;
-      tc_fence_after();
-      OutT* crow = C + static_cast<long long>(row) * ldc;
+    uint8_t* out = smem + Cfg::kRingBytes + q * Cfg::kOutBufs * Cfg::kOutBytes;
+    int buf = 0;
+    uint32_t acc = 0, uses = 0;
+    bool ok = true;
+    for (int t = first; ok && t < pl.items; t += step) {
+      const PairItem it = pair_item(pl, t, N);
+      const int row0 = it.m0 + rank * 128 + q * 32, row = row0 + lane;
+      for (int half = 0; half < it.halves; ++half) {
+        const int col0 = it.c0 + half * pl.n, cols = min(pl.n, N - col0);
+        OutT* crow = C + static_cast<long long>(row) * ldc;
+        uint4 old[ACCUM && sizeof(OutT) == 2 ? 32 : 1];
+        if constexpr (ACCUM && sizeof(OutT) == 2) {
+          // what is added to comes while the products are formed (N is a multiple of 8 here)
+          if (by_tma && row < M) {
+#pragma unroll
+            for (int v = 0; v < 32; ++v)
+              if (v * 8 < cols) old[v] = *reinterpret_cast<const uint4*>(crow + col0 + v * 8);
+          }
+        }
+        ok = mbar_wait_warp(&tmem_full_bar[acc], uses & 1, &cta_abort, status);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * 256;
+        if (by_tma) {
+#pragma unroll
+          for (int c = 0; c < 256 / kCols; ++c) {
+            if (c * kCols < cols) {
+              uint32_t r[kCols];
+#pragma unroll
+              for (int i = 0; i < kCols; i += 32) tmem_ld_32x32(addr + c * kCols + i, *reinterpret_cast<uint32_t(*)[32]>(&r[i]));
+              tmem_ld_wait();
+              if (lane == 0) tma_store_wait_read<Cfg::kOutBufs - 1>();       // the store that last read this buffer
+              __syncwarp();
+              uint8_t* piece = out + buf * Cfg::kOutBytes;
+#pragma unroll
+              for (int v = 0; v < 8; ++v) {
+                uint4 o;
+                if constexpr (sizeof(OutT) == 2) {
+                  float f[8];
+#pragma unroll
+                  for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(r[v * 8 + j]);
+                  if constexpr (ACCUM) {
+                    const __nv_bfloat162* o2 = reinterpret_cast<const __nv_bfloat162*>(&old[c * 8 + v]);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                      const float2 of = __bfloat1622float2(o2[j]);
+                      f[2 * j] += of.x;
+                      f[2 * j + 1] += of.y;
+                    }
+                  }
+                  o = make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+                } else {
+                  o = make_uint4(r[v * 4], r[v * 4 + 1], r[v * 4 + 2], r[v * 4 + 3]);
+                }
+                *reinterpret_cast<uint4*>(piece + lane * 128 + ((v ^ (lane & 7)) << 4)) = o;
+              }
+              fence_proxy_async_smem();
+              __syncwarp();
+              if (lane == 0) {
+                if (row0 < M) tma_store_2d(&tmC, piece, col0 + c * kCols, row0);
+                tma_store_commit();
+              }
+              buf ^= 1;
+            }
+          }
+        } else {
 #pragma unroll 1
-      for (int c = 0; c < Cfg::BN2 / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * Cfg::BN2 + c * 32), r);
-        tmem_ld_wait();
-        const int col0 = n0 + c * 32;
-        if (row < M && col0 < N) store_columns<OutT, ACCUM>(crow, col0, N, vec_ok, r, false, false);
+          for (int c = 0; c < pl.n / 32; ++c) {
+            uint32_t r[32];
+            tmem_ld_32x32(addr + c * 32, r);
+            tmem_ld_wait();
+            if (row < M && c * 32 < cols) store_columns<OutT, ACCUM>(crow, col0 + c * 32, N, vec_ok, r, false, false);
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(in_first_cta(&tmem_empty_bar[acc]));
+        uses += acc;
+        acc ^= 1;
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(in_first_cta(&tmem_empty_bar[acc]));
-      acc ^= 1;
-      if (acc == 0) acc_phase ^= 1u;
     }
+    if (lane == 0) tma_store_wait_all<0>();
   }
 
   // ------------------------------------------------------------ tear-down
@@ -598,9 +764,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 struct TmapKey {
   const void* p;
   uint64_t rows, cols, stride;
-  uint32_t br, bc;
+  uint32_t br, bc, elem;
   bool operator==(const TmapKey& o) const {
-    return p == o.p && rows == o.rows && cols == o.cols && stride == o.stride && br == o.br && bc == o.bc;
+    return p == o.p && rows == o.rows && cols == o.cols && stride == o.stride && br == o.br && bc == o.bc && elem == o.elem;
   }
 };
 struct TmapKeyHash {
@@ -609,7 +775,7 @@ struct TmapKeyHash {
     h ^= k.rows * 0xC2B2AE3D27D4EB4Full + (h << 6) + (h >> 2);
     h ^= k.cols * 0x165667B19E3779F9ull + (h << 6) + (h >> 2);
     h ^= k.stride + (h << 6) + (h >> 2);
-    h ^= (static_cast<size_t>(k.br) << 32 | k.bc) + (h << 6) + (h >> 2);
+    h ^= (static_cast<size_t>(k.br) << 32 | k.bc << 4 | k.elem) + (h << 6) + (h >> 2);
     return h;
   }
 };
@@ -617,15 +783,15 @@ std::unordered_map<TmapKey, CUtensorMap, TmapKeyHash> g_tmaps;
 std::mutex g_tmap_mu;
 
 bool cached_tmap_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t stride_bytes,
-                    uint32_t box_rows, uint32_t box_cols) {
-  TmapKey key{base, rows, cols, stride_bytes, box_rows, box_cols};
+                    uint32_t box_rows, uint32_t box_cols, int elem_bytes = 2) {
+  TmapKey key{base, rows, cols, stride_bytes, box_rows, box_cols, static_cast<uint32_t>(elem_bytes)};
   std::lock_guard<std::mutex> lk(g_tmap_mu);
   auto it = g_tmaps.find(key);
   if (it != g_tmaps.end()) {
     *out = it->second;
     return true;
   }
-  if (!make_tmap_2d(out, base, 2, rows, cols, stride_bytes, box_rows, box_cols, true)) return false;
+  if (!make_tmap_2d(out, base, elem_bytes, rows, cols, stride_bytes, box_rows, box_cols, true)) return false;
   if (g_tmaps.size() > 8192) g_tmaps.clear();
   g_tmaps.emplace(key, *out);
   return true;
@@ -672,7 +838,7 @@ int launch_major(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int M, i
 }
 
 template <bool A_MN, bool B_MN, typename OutT, bool ACCUM>
-int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int M, int N, int K, long long ldc, cudaStream_t stream) {
+int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int M, int N, int K, long long ldc, const PairPlan& plan, cudaStream_t stream) {
   auto kern = gemm_pair_kernel<A_MN, B_MN, OutT, ACCUM>;
   static PerDeviceFlag attr_set;
   if (attr_set.unset()) {
@@ -680,20 +846,53 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int M, in
     if (e != cudaSuccess) return static_cast<int>(e);
     attr_set.set();
   }
-  const int tiles = ((M + PairTile::BM2 - 1) / PairTile::BM2) * ((N + PairTile::BN2 - 1) / PairTile::BN2), pairs = sm_count() / 2;
-  kern<<<2 * (tiles < pairs ? tiles : pairs), kGemmThreads, PairTile::kSmemBytes, stream>>>(ta, tb, static_cast<OutT*>(C), M, N, K, ldc,
-                                                                                          device_status_word());
+  // Stores by TMA want rows that start on 16 bytes. Added to (ACCUM), bf16 rows are also read 16 bytes at a time up to N, and fp32 rows,
+  // of which a thread cannot hold enough ahead, go the plain way.
+  CUtensorMap tc{};
+  const int by_tma = (reinterpret_cast<uintptr_t>(C) & 15) == 0 && ldc * sizeof(OutT) % 16 == 0 && (!ACCUM || (sizeof(OutT) == 2 && N % 8 == 0));
+  if (by_tma && !cached_tmap_2d(&tc, C, M, N, ldc * sizeof(OutT), 32, 128 / sizeof(OutT), sizeof(OutT))) return -3;
+  const int pairs = sm_count() / 2;
+  kern<<<2 * (plan.items < pairs ? plan.items : pairs), kGemmThreads, PairTile::kSmemBytes, stream>>>(
+      ta, tb, tc, static_cast<OutT*>(C), M, N, K, ldc, plan, by_tma, device_status_word());
   return static_cast<int>(cudaGetLastError());
 }
 
 template <bool A_MN, bool B_MN>
 int launch_pair_out(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int M, int N, int K, long long ldc, int out_f32, int accumulate,
-                    cudaStream_t s) {
+                    const PairPlan& pl, cudaStream_t s) {
   if (out_f32)
-    return accumulate ? launch_pair<A_MN, B_MN, float, true>(ta, tb, C, M, N, K, ldc, s)
-                      : launch_pair<A_MN, B_MN, float, false>(ta, tb, C, M, N, K, ldc, s);
-  return accumulate ? launch_pair<A_MN, B_MN, __nv_bfloat16, true>(ta, tb, C, M, N, K, ldc, s)
-                    : launch_pair<A_MN, B_MN, __nv_bfloat16, false>(ta, tb, C, M, N, K, ldc, s);
+    return accumulate ? launch_pair<A_MN, B_MN, float, true>(ta, tb, C, M, N, K, ldc, pl, s)
+                      : launch_pair<A_MN, B_MN, float, false>(ta, tb, C, M, N, K, ldc, pl, s);
+  return accumulate ? launch_pair<A_MN, B_MN, __nv_bfloat16, true>(ta, tb, C, M, N, K, ldc, pl, s)
+                    : launch_pair<A_MN, B_MN, __nv_bfloat16, false>(ta, tb, C, M, N, K, ldc, pl, s);
+}
+
+PairPlan make_pair_plan(int M, int N, int n, int per) {
+  const int num_m = (M + 255) / 256, num_w = (N + per * n - 1) / (per * n);
+  const int tiles = num_m * num_w, pairs = sm_count() / 2, rest = tiles % pairs;
+  const int full = per == 2 && 2 * rest <= pairs ? tiles - rest : tiles;
+  // rows of tiles that are worked on together: with few columns of tiles a round covers all of them (17000 x 4096 x 14336: 8 1473, 16 1485 us),
+  // with many, more rows keep what it reads small (8192 x 28672 x 4096: 16 1412, 8 1435)
+  return {n, per, num_w >= 16 ? 16 : 8, num_m, num_w, full, full + 2 * (tiles - full)};
+}
+
+// What a product takes with tiles of a kind, up to a factor that they share: the tiles that one SM (or pair) works on in turn, times the
+// columns of a tile, times how much slower a column is than in the widest ones. The figures are times of 35 products of training and
+// prompts (64 - 18944 rows, depths 128 - 28672), all kinds of tiles in turn. Deep products want whole tiles of 256 x 512 (8192 x 4096 x 28672:
+// 1393 us against 1475 for halves by themselves; 4096 deep the same), shallow ones halves, whose stores start earlier (3003 x 16384 x 2048: 163
+// against 166). Widths of 192 fit where 256 would leave most of a round empty (3003 x 2048 x 8192: 72 against 93). Tiles of one SM remain for
+// up to 128 rows, for few tiles (296 x 2176 x 5120: 64 columns 18.5, pairs 23.8 at best) and where the last pair of row tiles would be half
+// empty (528 x 44384 x 3264: 142 against 166).
+double pair_cost(const PairPlan& pl, int K) {
+  const int pairs = sm_count() / 2, halves = pl.items - pl.full;
+  const int rounds = (pl.full + pairs - 1) / pairs * pl.per + (halves > 0 ? 1 : 0);
+  const double slow = (pl.per == 2 ? 1.0 : K >= 6144 ? 1.05 : K >= 3072 ? 1.0 : 0.95) *
+                      (pl.n == 256 ? 1.0 : pl.n == 128 ? 1.25 : pl.per == 2 ? 1.04 : 1.08);
+  return rounds * pl.n * slow;
+}
+double cta_cost(int M, int N, int K, int bn) {
+  const long long tiles = static_cast<long long>((M + BM - 1) / BM) * ((N + bn - 1) / bn);
+  return static_cast<double>((tiles + sm_count() - 1) / sm_count()) * bn * (bn == 256 ? (K >= 3072 ? 1.06 : 1.15) : bn == 128 ? 1.33 : bn == 64 ? 2.25 : 4.0);
 }
 
 }  // namespace
@@ -717,19 +916,11 @@ TSB_EXPORT int tsb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
     return -2;
   int bn = block_n;
   bool pair = false;
+  PairPlan plan{};
   if (bn == 0) {
     const int sms = sm_count();
     const long long mt = (M + BM - 1) / BM;
     auto tiles = [&](int b) { return mt * ((N + b - 1) / b); };
-    // 128 x 256 tiles would be chosen, and tiles of 256 x 256 for pairs of SMs take no more rounds than they. Time of the former over that of
-    // the latter, sustained: K = 256 0.82, 512 0.98, 768 0.96 - 1.01, 896 0.97 - 1.07, 960 1.08, 1024 - 1536 1.00 - 1.14 (9001 x 1288 x 1000
-    // 1.21), 2048 - 8192 1.00 - 1.08 (two rounds of which the second is a third full 1.00, 8192 x 28672 x 4096 1.05), 9216 - 12288 1.00 - 1.02.
-    // Beyond, 1.00 - 1.06 where the rows of both operands run along M and N (weight gradients: 4096 x 4096 x 16384 1.04), else 0.975 - 1.01
-    // (4096 x 4096 x 128256 0.975, 4096 x 4096 x 32768 0.98, 17408 1.007). (Runs of one side differ by 1 %.)
-    if (max_ctas <= 0 && N >= 256 && tiles(256) >= sms && K >= 960 && (K <= 12288 || (a_mn && b_mn))) {
-      const long long pairs = sms / 2, tiles2 = ((M + 255) / 256) * static_cast<long long>((N + 255) / 256);
-      pair = (tiles2 + pairs - 1) / pairs <= (tiles(256) + sms - 1) / sms;
-    }
     // largest tile that still gives every SM work; decode-shaped calls (few rows) stream the weight matrix
     // and want as many CTAs pulling on HBM as possible, so they go down to 32-column tiles
     if (N >= 256 && tiles(256) >= sms) bn = 256;
@@ -737,6 +928,24 @@ TSB_EXPORT int tsb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
     else if (N >= 64 && tiles(64) >= sms) bn = 64;
     else if (N >= 128 && tiles(128) * 2 >= sms && mt > 2) bn = 128;
     else bn = (N >= 64 && tiles(32) > 2 * sms) ? 64 : 32;
+    // More than one tile of rows, and columns for a wide one: the cheapest kind.
+    if (max_ctas <= 0 && M > 128 && N >= 192) {
+      double best = cta_cost(M, N, K, bn);
+      for (const int b : {64, 128, 256})
+        if (const double cost = cta_cost(M, N, K, b); cost < best) {
+          best = cost;
+          bn = b;
+        }
+      constexpr int kinds[][2] = {{256, 2}, {256, 1}, {192, 2}, {192, 1}, {128, 1}};
+      for (const auto& kind : kinds) {
+        const PairPlan pl = make_pair_plan(M, N, kind[0], kind[1]);
+        if (const double cost = pair_cost(pl, K); cost < best) {
+          best = cost;
+          plan = pl;
+          pair = true;
+        }
+      }
+    }
   }
   if (bn == 32 && b_mn) bn = 64;  // an N-major B tile is built from 64-column (128-byte) boxes
   if (bn != 32 && bn != 64 && bn != 128 && bn != 256) return -2;
@@ -745,16 +954,16 @@ TSB_EXPORT int tsb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
   if (!a_mn) ok = cached_tmap_2d(&ta, A, M, K, lda * 2, BM, BK);
   else ok = cached_tmap_2d(&ta, A, K, M, lda * 2, BK, 64);
   if (!ok) return -3;
-  if (!b_mn) ok = cached_tmap_2d(&tb, B, N, K, ldb * 2, pair ? 128 : bn, BK);
+  if (!b_mn) ok = cached_tmap_2d(&tb, B, N, K, ldb * 2, pair ? plan.n / 2 : bn, BK);
   else ok = cached_tmap_2d(&tb, B, K, N, ldb * 2, BK, 64);
   if (!ok) return -3;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (pair) {
     if (!a_mn)
-      return b_mn ? launch_pair_out<false, true>(ta, tb, C, M, N, K, ldc, out_f32, accumulate, s)
-                  : launch_pair_out<false, false>(ta, tb, C, M, N, K, ldc, out_f32, accumulate, s);
-    return b_mn ? launch_pair_out<true, true>(ta, tb, C, M, N, K, ldc, out_f32, accumulate, s)
-                : launch_pair_out<true, false>(ta, tb, C, M, N, K, ldc, out_f32, accumulate, s);
+      return b_mn ? launch_pair_out<false, true>(ta, tb, C, M, N, K, ldc, out_f32, accumulate, plan, s)
+                  : launch_pair_out<false, false>(ta, tb, C, M, N, K, ldc, out_f32, accumulate, plan, s);
+    return b_mn ? launch_pair_out<true, true>(ta, tb, C, M, N, K, ldc, out_f32, accumulate, plan, s)
+                : launch_pair_out<true, false>(ta, tb, C, M, N, K, ldc, out_f32, accumulate, plan, s);
   }
   switch (bn) {
     case 256: return launch_major<256>(ta, tb, C, M, N, K, ldc, a_mn, b_mn, out_f32, accumulate, max_ctas, s);

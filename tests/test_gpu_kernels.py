@@ -496,6 +496,32 @@ def test_gemm_tiles_of_two_sms(dev, M, N, K, pad, a_mn, b_mn, out, accumulate):
     assert torch.equal(rows[:, N:], beside)
 
 
+@pytest.mark.parametrize("M,N,K,pad", [(3000, 6392, 6152, 0), (3000, 6392, 6152, 3),   # tiles of 256 x 512, the rest as halves, some beyond N
+                                       (2600, 2048, 8200, 0),                          # 256 x 384 whole
+                                       (3000, 2048, 2056, 0), (1072, 1152, 3264, 0),   # halves of 192, of 128
+                                       (2600, 12104, 72, 0)])                          # of 256, two blocks of K
+@pytest.mark.parametrize("a_mn", [False, True])
+@pytest.mark.parametrize("b_mn", [False, True])
+@pytest.mark.parametrize("out,accumulate", [(torch.bfloat16, False), (torch.bfloat16, True), (torch.float32, False)])
+def test_gemm_kinds_of_tiles(dev, M, N, K, pad, a_mn, b_mn, out, accumulate):
+    """Every kind of tile of two SMs at its edges, stored by TMA or (rows off 16 bytes) directly. Bounds as above; a wrong column or row of
+    a tile would stand out by the size of the result."""
+    from tesseract_b200.ops.gemm import gemm_bf16
+    g = torch.Generator(device=dev).manual_seed(M + N + K)
+    a = torch.randn(*((K, M) if a_mn else (M, K)), device=dev, generator=g).bfloat16()
+    b = torch.randn(*((K, N) if b_mn else (N, K)), device=dev, generator=g).bfloat16()
+    rows = torch.randn(M, N + pad, device=dev, generator=g).to(out)
+    beside, c = rows[:, N:].clone(), rows[:, :N]
+    ref = (a.t() if a_mn else a).double() @ (b if b_mn else b.t()).double() + (c.double() if accumulate else 0)
+    gemm_bf16(a, b, a_mn=a_mn, b_mn=b_mn, out=c, accumulate=accumulate)
+    torch.cuda.synchronize()
+    _status_ok()
+    assert float((c.double() - ref).norm() / ref.norm()) < (3e-3 if out == torch.bfloat16 else 1e-4)
+    # a value's error: half a step of bf16, 2^-9 of the largest, or what fp32 sums of this depth leave
+    assert float((c.double() - ref).abs().max()) <= float(ref.abs().max()) * (2.0 ** -8 if out == torch.bfloat16 else 1e-4)
+    assert torch.equal(rows[:, N:], beside)
+
+
 @pytest.mark.parametrize("H,Hkv", [(4, 2), (3, 3), (6, 2)])       # two heads of a group per CTA; two tiles of a head
 @pytest.mark.parametrize("Sq,Sk", [(1, 1), (1, 300), (127, 127), (128, 128), (129, 640), (257, 257), (300, 200)])
 @pytest.mark.parametrize("D", [64, 128])
