@@ -103,7 +103,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   __shared__ uint32_t tmem_base_smem;
   __shared__ volatile int cta_abort;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
   // KV heads on the fast axis: under causal masking the first key tiles, seen by the most queries, all start first. (Both on x: key
   // tiles may be more than the other axes take.)
@@ -169,81 +169,90 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     warpgroup_regs_dec<kBwdOtherRegs>();
     if (warp == 12) {
       // ---------------------------------------------------------------- TMA producer
-      if (lane == 0 && n_iter > 0) {
-        mbar_expect_tx(&kv_full, 2 * Cfg::kTileBytes);
+      if (n_iter > 0) {
+        const bool lead = elect_one();       // (the loops of warps 12 and 13 are walked by the whole warp)
+        if (lead) {
+          mbar_expect_tx(&kv_full, 2 * Cfg::kTileBytes);
 #pragma unroll
-        for (int hf = 0; hf < Cfg::kHalves; ++hf) {
-          tma_load_4d(sK + hf * 16384, &tmK, &kv_full, hf * 64, c0, hk, b);
-          tma_load_4d(sV + hf * 16384, &tmV, &kv_full, hf * 64, c0, hk, b);
+          for (int hf = 0; hf < Cfg::kHalves; ++hf) {
+            tma_load_4d(sK + hf * 16384, &tmK, &kv_full, hf * 64, c0, hk, b);
+            tma_load_4d(sV + hf * 16384, &tmV, &kv_full, hf * 64, c0, hk, b);
+          }
         }
         Walk w = first;
         for (int t = 0; t < n_iter; ++t, next(w)) {
           const int i = w.i, h = w.h;
           const int qs = t % Cfg::kQStages, ds = t % Cfg::kDOStages;
-          if (!mbar_wait(&q_empty[qs], ((t / Cfg::kQStages) & 1) ^ 1u, &cta_abort, p.status)) break;
+          if (!mbar_wait_warp(&q_empty[qs], ((t / Cfg::kQStages) & 1) ^ 1u, &cta_abort, p.status)) break;
           const long long at = ((static_cast<long long>(b) * p.H + h) * p.n_q + i) * BT;
-          mbar_expect_tx(&q_full[qs], Cfg::kTileBytes + Cfg::kRowBytes);
+          if (lead) {
+            mbar_expect_tx(&q_full[qs], Cfg::kTileBytes + Cfg::kRowBytes);
 #pragma unroll
-          for (int hf = 0; hf < Cfg::kHalves; ++hf)
-            tma_load_4d(sQ + qs * Cfg::kTileBytes + hf * 16384, &tmQ, &q_full[qs], hf * 64, i * BT, h, b);
-          bulk_load(sRow + qs * Cfg::kRowBytes, p.lse2 + at, BT * 4, &q_full[qs]);
-          bulk_load(sRow + qs * Cfg::kRowBytes + BT * 4, p.delta + at, BT * 4, &q_full[qs]);
-          if (!mbar_wait(&do_empty[ds], ((t / Cfg::kDOStages) & 1) ^ 1u, &cta_abort, p.status)) break;
-          mbar_expect_tx(&do_full[ds], Cfg::kTileBytes);
+            for (int hf = 0; hf < Cfg::kHalves; ++hf)
+              tma_load_4d(sQ + qs * Cfg::kTileBytes + hf * 16384, &tmQ, &q_full[qs], hf * 64, i * BT, h, b);
+            bulk_load(sRow + qs * Cfg::kRowBytes, p.lse2 + at, BT * 4, &q_full[qs]);
+            bulk_load(sRow + qs * Cfg::kRowBytes + BT * 4, p.delta + at, BT * 4, &q_full[qs]);
+          }
+          if (!mbar_wait_warp(&do_empty[ds], ((t / Cfg::kDOStages) & 1) ^ 1u, &cta_abort, p.status)) break;
+          if (lead) {
+            mbar_expect_tx(&do_full[ds], Cfg::kTileBytes);
 #pragma unroll
-          for (int hf = 0; hf < Cfg::kHalves; ++hf)
-            tma_load_4d(sDO + ds * Cfg::kTileBytes + hf * 16384, &tmDO, &do_full[ds], hf * 64, i * BT, h, b);
+            for (int hf = 0; hf < Cfg::kHalves; ++hf)
+              tma_load_4d(sDO + ds * Cfg::kTileBytes + hf * 16384, &tmDO, &do_full[ds], hf * 64, i * BT, h, b);
+          }
+          __syncwarp();
         }
       }
     } else if (warp == 13) {
       // ---------------------------------------------------------------- MMA issuer
-      if (lane == 0 && n_iter > 0) {
+      if (n_iter > 0) {
+        const uint32_t lead = elect_one() ? 1u : 0u;
         constexpr uint32_t idesc_s = umma_idesc(BT, BT, 1, 1, 0, 0);   // S^T, dP^T: both operands K-major
         constexpr uint32_t idesc_kv = umma_idesc(BT, D, 1, 1, 0, 1);   // dV, dK: P^T / dS^T in TMEM, dO / Q N-major
         constexpr uint32_t idesc_q = umma_idesc(BT, D, 1, 1, 1, 1);    // dQ: dS M-major, K N-major
         const uint32_t k_base = smem_u32(sK), v_base = smem_u32(sV), ds_base = smem_u32(sDS);
         auto scores = [&](int t) -> bool {
           const int qs = t % Cfg::kQStages;
-          if (!mbar_wait(&q_full[qs], (t / Cfg::kQStages) & 1, &cta_abort, p.status)) return false;
+          if (!mbar_wait_warp(&q_full[qs], (t / Cfg::kQStages) & 1, &cta_abort, p.status)) return false;
           tc_fence_after();
           const uint32_t q_base = smem_u32(sQ + qs * Cfg::kTileBytes);
 #pragma unroll
           for (int ks = 0; ks < D / 16; ++ks)
-            umma_f16(tmem_base + Cfg::kColS, kmajor_desc<128>(k_base, ks), kmajor_desc<128>(q_base, ks), idesc_s, ks != 0);
-          umma_commit(&s_full);
+            umma_f16_if(lead, tmem_base + Cfg::kColS, kmajor_desc<128>(k_base, ks), kmajor_desc<128>(q_base, ks), idesc_s, ks != 0);
+          umma_commit_if(lead, &s_full);
           return true;
         };
-        bool ok = mbar_wait(&kv_full, 0, &cta_abort, p.status) && scores(0);
+        bool ok = mbar_wait_warp(&kv_full, 0, &cta_abort, p.status) && scores(0);
         for (int t = 0; ok && t < n_iter; ++t) {
           const uint32_t ph = t & 1;
           const uint32_t q_base = smem_u32(sQ + (t % Cfg::kQStages) * Cfg::kTileBytes);
           const uint32_t do_base = smem_u32(sDO + (t % Cfg::kDOStages) * Cfg::kTileBytes);
-          if (!mbar_wait(&do_full[t % Cfg::kDOStages], (t / Cfg::kDOStages) & 1, &cta_abort, p.status)) break;
-          if (!mbar_wait(&dq_read, ph ^ 1u, &cta_abort, p.status)) break;
+          if (!mbar_wait_warp(&do_full[t % Cfg::kDOStages], (t / Cfg::kDOStages) & 1, &cta_abort, p.status)) break;
+          if (!mbar_wait_warp(&dq_read, ph ^ 1u, &cta_abort, p.status)) break;
           tc_fence_after();
 #pragma unroll
           for (int ks = 0; ks < D / 16; ++ks)    // dP^T = V dO^T
-            umma_f16(tmem_base + Cfg::kColDP, kmajor_desc<128>(v_base, ks), kmajor_desc<128>(do_base, ks), idesc_s, ks != 0);
-          umma_commit(&dp_full);
-          if (!mbar_wait(&p_full, ph, &cta_abort, p.status)) break;
+            umma_f16_if(lead, tmem_base + Cfg::kColDP, kmajor_desc<128>(v_base, ks), kmajor_desc<128>(do_base, ks), idesc_s, ks != 0);
+          umma_commit_if(lead, &dp_full);
+          if (!mbar_wait_warp(&p_full, ph, &cta_abort, p.status)) break;
           tc_fence_after();
 #pragma unroll
           for (int ks = 0; ks < BT / 16; ++ks)   // dV += P^T dO   (K = query rows; each half of P^T lies over its half of S^T)
-            umma_f16_ts(tmem_base + Cfg::kColDV, tmem_base + Cfg::kColS + (ks >> 2) * 64 + (ks & 3) * 8, mnmajor_desc(do_base, ks, 16384),
+            umma_f16_ts_if(lead, tmem_base + Cfg::kColDV, tmem_base + Cfg::kColS + (ks >> 2) * 64 + (ks & 3) * 8, mnmajor_desc(do_base, ks, 16384),
                         idesc_kv, (t | ks) != 0);
-          umma_commit(&do_empty[t % Cfg::kDOStages]);
+          umma_commit_if(lead, &do_empty[t % Cfg::kDOStages]);
           if (t + 1 < n_iter && !scores(t + 1)) break;
-          if (!mbar_wait(&ds_full, ph, &cta_abort, p.status)) break;
+          if (!mbar_wait_warp(&ds_full, ph, &cta_abort, p.status)) break;
           tc_fence_after();
 #pragma unroll
           for (int ks = 0; ks < BT / 16; ++ks)   // dK += dS^T Q
-            umma_f16_ts(tmem_base + Cfg::kColDK, tmem_base + Cfg::kColDP + (ks >> 2) * 64 + (ks & 3) * 8, mnmajor_desc(q_base, ks, 16384),
+            umma_f16_ts_if(lead, tmem_base + Cfg::kColDK, tmem_base + Cfg::kColDP + (ks >> 2) * 64 + (ks & 3) * 8, mnmajor_desc(q_base, ks, 16384),
                         idesc_kv, (t | ks) != 0);
 #pragma unroll
           for (int ks = 0; ks < BT / 16; ++ks)   // dQ = dS K       (K = key rows; with 128 columns over dS^T, which dK has read)
-            umma_f16(tmem_base + Cfg::kColDQ, mnmajor_desc(ds_base, ks, 16384), mnmajor_desc(k_base, ks, 16384), idesc_q, ks != 0);
-          umma_commit(&dq_full);
-          umma_commit(&q_empty[t % Cfg::kQStages]);
+            umma_f16_if(lead, tmem_base + Cfg::kColDQ, mnmajor_desc(ds_base, ks, 16384), mnmajor_desc(k_base, ks, 16384), idesc_q, ks != 0);
+          umma_commit_if(lead, &dq_full);
+          umma_commit_if(lead, &q_empty[t % Cfg::kQStages]);
         }
       }
     }

@@ -765,7 +765,7 @@ flash_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   __shared__ __align__(8) uint64_t q_full[2], kv_full[Cfg::kSlots], kv_empty[Cfg::kSlots], s_full[2], s_read[2], p_half[2], p_full[2], o_full[2];
   __shared__ uint32_t tmem_base_smem;
   __shared__ volatile int cta_abort;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     cta_abort = 0;
     for (int i = 0; i < 2; ++i) {
@@ -798,44 +798,47 @@ flash_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     warpgroup_regs_dec<kPairOtherRegs>();
     if (warp == 8) {
       // ---------------------------------------------------------------- TMA producer: tile 2 j is K_j, tile 2 j + 1 is V_j
-      if (lane == 0) {
-        auto load_q = [&](int s) {
-          if (n_of[s] == 0) return;
-          mbar_expect_tx(&q_full[s], Cfg::kTileBytes);
+      const bool lead = elect_one();         // (the loops of warps 8 - 10 are walked by the whole warp)
+      auto load_q = [&](int s) {
+        if (n_of[s] == 0 || !lead) return;
+        mbar_expect_tx(&q_full[s], Cfg::kTileBytes);
 #pragma unroll
-          for (int hf = 0; hf < Cfg::kHalves; ++hf)
-            tma_load_4d(sQ + s * Cfg::kTileBytes + hf * 16384, &tmQ, &q_full[s], hf * 64, row0 + qa + (pair_heads ? 0 : s * BQ),
-                        ha + (pair_heads ? s : 0), bb);
-        };
-        load_q(0);
-        for (int t = 0; t < 2 * n_tiles; ++t) {
-          const int st = t % Cfg::kSlots;
-          if (!mbar_wait(&kv_empty[st], ((t / Cfg::kSlots) & 1) ^ 1u, &cta_abort, p.status)) break;
+        for (int hf = 0; hf < Cfg::kHalves; ++hf)
+          tma_load_4d(sQ + s * Cfg::kTileBytes + hf * 16384, &tmQ, &q_full[s], hf * 64, row0 + qa + (pair_heads ? 0 : s * BQ),
+                      ha + (pair_heads ? s : 0), bb);
+      };
+      load_q(0);
+      for (int t = 0; t < 2 * n_tiles; ++t) {
+        const int st = t % Cfg::kSlots;
+        if (!mbar_wait_warp(&kv_empty[st], ((t / Cfg::kSlots) & 1) ^ 1u, &cta_abort, p.status)) break;
+        if (lead) {
           mbar_expect_tx(&kv_full[st], Cfg::kTileBytes);
 #pragma unroll
           for (int hf = 0; hf < Cfg::kHalves; ++hf)
             tma_load_4d(sKV + st * Cfg::kTileBytes + hf * 16384, t & 1 ? &tmV : &tmK, &kv_full[st], hf * 64, (t >> 1) * BKV + krow0, hk, bb);
-          if (t == 0) load_q(1);
         }
+        if (t == 0) load_q(1);
+        __syncwarp();
       }
     } else if (warp <= 10) {
       // ---------------------------------------------------------------- MMA issuers
-      if (lane == 0 && n_tiles > 0 && (Cfg::kOwnP || warp == 9)) {
+      if (n_tiles > 0 && (Cfg::kOwnP || warp == 9)) {
+        const uint32_t lead = elect_one() ? 1u : 0u;
         constexpr uint32_t idesc_s = umma_idesc(BQ, BKV, 1, 1, 0, 0);  // S = Q K^T, both K-major
         constexpr uint32_t idesc_o = umma_idesc(BQ, D, 1, 1, 0, 1);    // O += P V, P in TMEM, V N-major
         const int n0 = n_of[0], n1 = n_of[1];
         const uint32_t q_base = smem_u32(sQ), kv_base = smem_u32(sKV);
-        auto slot_full = [&](int t) { return mbar_wait(&kv_full[t % Cfg::kSlots], (t / Cfg::kSlots) & 1, &cta_abort, p.status); };
+        auto slot_full = [&](int t) { return mbar_wait_warp(&kv_full[t % Cfg::kSlots], (t / Cfg::kSlots) & 1, &cta_abort, p.status); };
         auto scores = [&](int s, int j) {
           const uint32_t k_base = kv_base + ((2 * j) % Cfg::kSlots) * Cfg::kTileBytes;
 #pragma unroll
           for (int ks = 0; ks < D / 16; ++ks)
-            umma_f16(tmem_base + s * BKV, kmajor_desc<128>(q_base + s * Cfg::kTileBytes, ks), kmajor_desc<128>(k_base, ks), idesc_s, ks != 0);
-          umma_commit(&s_full[s]);
+            umma_f16_if(lead, tmem_base + s * BKV, kmajor_desc<128>(q_base + s * Cfg::kTileBytes, ks), kmajor_desc<128>(k_base, ks), idesc_s, ks != 0);
+          umma_commit_if(lead, &s_full[s]);
         };
         auto begin = [&](int s) -> bool {
           if ((s ? n1 : n0) == 0) return true;
-          if (!mbar_wait(&q_full[s], 0, &cta_abort, p.status)) return false;
+          if (!mbar_wait_warp(&q_full[s], 0, &cta_abort, p.status)) return false;
           tc_fence_after();
           scores(s, 0);
           return true;
@@ -844,7 +847,7 @@ flash_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         auto next_scores = [&](int s, int j) -> bool {
           if (j + 1 >= (s ? n1 : n0)) return true;
           if (Cfg::kOwnP) {
-            if (!mbar_wait(&s_read[s], j & 1, &cta_abort, p.status)) return false;
+            if (!mbar_wait_warp(&s_read[s], j & 1, &cta_abort, p.status)) return false;
             tc_fence_after();
           }
           scores(s, j + 1);                  // heads of 128: over P, which the MMAs before it have read by then
@@ -856,39 +859,39 @@ flash_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           // P V of the first 64 keys starts while the exponentials of the others are taken
 #pragma unroll
           for (int part = 0; part < 2; ++part) {
-            if (!mbar_wait(part ? &p_full[s] : &p_half[s], j & 1, &cta_abort, p.status)) return false;
+            if (!mbar_wait_warp(part ? &p_full[s] : &p_half[s], j & 1, &cta_abort, p.status)) return false;
             tc_fence_after();
 #pragma unroll
             for (int ks = part * 4; ks < part * 4 + 4; ++ks)
-              umma_f16_ts(tmem_base + Cfg::kColO + s * D, tmem_base + Cfg::kColP + s * Cfg::kPStride + ks * 8,
+              umma_f16_ts_if(lead, tmem_base + Cfg::kColO + s * D, tmem_base + Cfg::kColP + s * Cfg::kPStride + ks * 8,
                           mnmajor_desc(kv_base + ((2 * j + 1) % Cfg::kSlots) * Cfg::kTileBytes, ks, 16384), idesc_o, (j | ks) != 0);
           }
-          if (Cfg::kOwnP || j + 1 == n_own) umma_commit(&o_full[s]);
+          if (Cfg::kOwnP || j + 1 == n_own) umma_commit_if(lead, &o_full[s]);
           return true;
         };
         bool ok = slot_full(0);
         if constexpr (Cfg::kOwnP) {
           const int s = warp - 9;
           ok = ok && begin(s);
-          if (ok) umma_commit(&kv_empty[0]);
+          if (ok) umma_commit_if(lead, &kv_empty[0]);
           for (int j = 0; ok && j < n_tiles; ++j) {
             if (j + 1 < n_tiles) {
               ok = slot_full(2 * j + 2) && next_scores(s, j);
               if (!ok) break;
-              umma_commit(&kv_empty[(2 * j + 2) % Cfg::kSlots]);
+              umma_commit_if(lead, &kv_empty[(2 * j + 2) % Cfg::kSlots]);
             }
             ok = slot_full(2 * j + 1) && values(s, j);
-            if (ok) umma_commit(&kv_empty[(2 * j + 1) % Cfg::kSlots]);
+            if (ok) umma_commit_if(lead, &kv_empty[(2 * j + 1) % Cfg::kSlots]);
           }
         } else {
           ok = ok && begin(0) && begin(1);
-          if (ok) umma_commit(&kv_empty[0]);
+          if (ok) umma_commit_if(lead, &kv_empty[0]);
           for (int j = 0; ok && j < n_tiles; ++j) {
             const bool more = j + 1 < n_tiles;
             ok = slot_full(2 * j + 1) && (!more || slot_full(2 * j + 2)) && values(0, j) && next_scores(0, j) && values(1, j) && next_scores(1, j);
             if (!ok) break;
-            umma_commit(&kv_empty[(2 * j + 1) % Cfg::kSlots]);
-            if (more) umma_commit(&kv_empty[(2 * j + 2) % Cfg::kSlots]);
+            umma_commit_if(lead, &kv_empty[(2 * j + 1) % Cfg::kSlots]);
+            if (more) umma_commit_if(lead, &kv_empty[(2 * j + 2) % Cfg::kSlots]);
           }
         }
       }
