@@ -171,4 +171,8 @@ def dtype_code(dtype) -> int:
 def stream_ptr(device=None) -> int:
     import torch
 
-    return torch.cuda.current_stream(device).cuda_stream
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)      # (a tenth of the time of building the Stream object)
+    index = device.index if isinstance(device, torch.device) else device
+    if raw is None or not isinstance(index, int):
+        return torch.cuda.current_stream(device).cuda_stream
+    return raw(index)

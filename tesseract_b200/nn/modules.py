@@ -371,6 +371,10 @@ class FeedForward(Module):
             self.replace_module(name, quantize_linear(getattr(self, name), scheme))
 
 
+_GLOBAL_HOOKS = tuple(n for n in ("_global_forward_hooks", "_global_forward_pre_hooks", "_global_backward_hooks", "_global_backward_pre_hooks")
+                      if hasattr(nn.modules.module, n))
+
+
 class TransformerBlock(Module):
     """Pre-norm block: h = x + attn(norm_1(x)); out = h + ffn(norm_2(h)) (src/nn/TransformerBlock.cpp:53-67).
 
@@ -388,7 +392,64 @@ class TransformerBlock(Module):
         self.norm_2 = RMSNorm(d_model, eps, dtype, device)
         self.ffn = ffn if ffn is not None else FeedForward(d_model, d_ff, dtype, device)
 
+    def _whole(self, x: torch.Tensor, residual: Optional[torch.Tensor]):
+        """Arguments of ``ops.decoder_block``, or None where the modules have to run one by one: anything but the classes of this file,
+        a hook on any of them, weights without a bf16 ``main_grad``, frozen or apart in memory, no gradient wanted, shapes or
+        settings that other kernels serve. Looked at in every pass: modules, weights and hooks may change between two."""
+        m1, attn, m2, ffn = (self._modules.get(n) for n in ("norm_1", "attn", "norm_2", "ffn"))
+        if not (x.is_cuda and x.dtype is torch.bfloat16 and x.requires_grad and torch.is_grad_enabled() and x.dim() == 3 and x.numel()
+                and type(m1) is RMSNorm and type(m2) is RMSNorm and type(attn) is MultiHeadAttention and type(ffn) is FeedForward):
+            return None
+        if residual is not None and (residual.shape != x.shape or residual.dtype is not x.dtype or residual.device != x.device):
+            return None
+        qkv = tuple(attn._modules.get(n) for n in ("q_proj", "k_proj", "v_proj"))
+        gu = tuple(ffn._modules.get(n) for n in ("gate_proj", "up_proj"))
+        o, down, rope = attn._modules.get("o_proj"), ffn._modules.get("down_proj"), attn.rope
+        linears = qkv + gu + (o, down)
+        if any(type(m) is not Linear or m._parameters.get("bias") is not None for m in linears) or type(rope) is not RotaryEmbedding:
+            return None
+        for m in (m1, attn, m2, ffn) + linears:
+            if (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__
+                    or "qkv" in m.__dict__):
+                return None
+        if any(getattr(nn.modules.module, n) for n in _GLOBAL_HOOKS):
+            return None
+        B, S, W = x.shape
+        H, Hkv, D, F = attn.num_heads, attn.num_kv_heads, attn.head_dim, ffn.d_ff
+        if D not in (64, 128) or H * D != W or H % Hkv or W > 8192 or F % 8 or B * S >= 1 << 30 or not ops.block_kernels_ok(x):
+            return None
+        shapes = {m1: (W,), m2: (W,), qkv[0]: (W, W), qkv[1]: (Hkv * D, W), qkv[2]: (Hkv * D, W), o: (W, W), gu[0]: (F, W), gu[1]: (F, W),
+                  down: (W, F)}
+        if len(shapes) != 9:
+            return None
+        weights, grads = {}, {}
+        for m, shape in shapes.items():
+            w = m._parameters.get("weight")
+            g = _main_grad(w)
+            if g is None or not w.requires_grad:
+                return None
+            for t in (w, g):
+                if (t.dtype is not torch.bfloat16 or t.shape != shape or t.device != x.device or not t.is_contiguous()
+                        or t.data_ptr() % 16):
+                    return None
+            weights[m], grads[m] = w, g
+        for group in (qkv, gu):
+            for a, b in zip(group[:-1], group[1:]):
+                for t in (weights, grads):
+                    if t[a].data_ptr() + 2 * t[a].numel() != t[b].data_ptr():
+                        return None
+        cos, sin = rope.cos, rope.sin
+        if any(t.dtype is not torch.float32 or t.device != x.device or not t.is_contiguous() or t.shape[0] < S or t.shape[1] != D // 2
+               for t in (cos, sin)):
+            return None
+        order = (m1, qkv[0], o, m2, gu[0], down)
+        return (x, residual, [weights[m] for m in order], [grads[m] for m in order], cos, sin, (B, S, W, H, Hkv, D, F),
+                (m1.eps, m2.eps, 1.0 / math.sqrt(D)), attn.causal)
+
     def forward_fused(self, x: torch.Tensor, residual: Optional[torch.Tensor]):
+        whole = self._whole(x, residual)
+        if whole is not None:
+            return ops.decoder_block(*whole)
         if residual is None:
             h, res = self.norm_1(x), x
         else:

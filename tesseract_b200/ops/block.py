@@ -1,0 +1,84 @@
+"""A pre-norm decoder block as one autograd function: the launches of ``rms_norm``, ``linear``, ``rope_qkv``, ``flash_attention_packed`` and
+``swiglu`` in the same order, issued by one native call per direction (``csrc/decoder_block.cu``). For training on CUDA with weights and
+gradients in an arena; ``nn.TransformerBlock`` decides when it stands for the modules that it takes the place of."""
+from __future__ import annotations
+
+import ctypes
+
+import torch
+
+from .. import _native
+from .._native import check, lib, stream_ptr
+from .attention import _native_flash_available
+from .gemm import _use_native
+
+_native.register_signatures({
+    "tsb_block_saved_bytes": [_native.P, _native.I],
+    "tsb_block_work_bytes": [_native.P],
+    "tsb_block_forward": [_native.P, _native.P, _native.P, _native.I, _native.P],
+    "tsb_block_backward": [_native.P, _native.P, _native.P, _native.I, _native.I, _native.P],
+})
+_native._RESTYPES["tsb_block_saved_bytes"] = _native._RESTYPES["tsb_block_work_bytes"] = _native.L
+
+_Shape, _Floats = ctypes.c_longlong * 7, ctypes.c_float * 3
+_Fwd, _Bwd = ctypes.c_longlong * 13, ctypes.c_longlong * 21
+LAUNCHES_FORWARD, LAUNCHES_BACKWARD = 9, 18
+
+
+def _ptr(t) -> int:
+    return 0 if t is None else t.data_ptr()
+
+
+def _rows(t: torch.Tensor) -> torch.Tensor:
+    """Contiguous rows that start on 16 bytes."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+class _BlockFn(torch.autograd.Function):
+    """(out, res2) of x and the residual stream. ``weights`` and ``grads``: norm_1, q / k / v, o, norm_2, gate / up, down; of the stacked
+    ones the first, which the others follow in memory."""
+
+    @staticmethod
+    def forward(ctx, x, res, norm_1, qkv, o, norm_2, gate_up, down, grads, cos, sin, shape, floats, causal):
+        ctx.set_materialize_grads(False)
+        x = _rows(x)
+        if res is not None:
+            res = _rows(res)
+        shape, floats = _Shape(*shape), _Floats(*floats)
+        saved = torch.empty(lib().tsb_block_saved_bytes(shape, int(res is not None)), device=x.device, dtype=torch.uint8)
+        res2, out = torch.empty_like(x), torch.empty_like(x)
+        weights = (norm_1, qkv, o, norm_2, gate_up, down)
+        args = _Fwd(x.data_ptr(), _ptr(res), *(w.data_ptr() for w in weights), cos.data_ptr(), sin.data_ptr(), saved.data_ptr(),
+                    res2.data_ptr(), out.data_ptr())
+        check(lib().tsb_block_forward(shape, args, floats, int(causal), stream_ptr(x.device)), "tsb_block_forward")
+        _native.add_launches(LAUNCHES_FORWARD - 1)
+        ctx.save_for_backward(x if res is None else None, res2, saved, cos, sin, *weights)
+        ctx.grads, ctx.has_res, ctx.args = grads, res is not None, (shape, floats, causal)
+        return out, res2
+
+    @staticmethod
+    def backward(ctx, dout, dres2):
+        x, res2, saved, cos, sin, *weights = ctx.saved_tensors
+        shape, floats, causal = ctx.args
+        dout = torch.zeros_like(res2) if dout is None else _rows(dout)
+        if dres2 is not None:
+            dres2 = _rows(dres2)
+        work = torch.empty(lib().tsb_block_work_bytes(shape), device=res2.device, dtype=torch.uint8)
+        dx = torch.empty_like(res2)
+        args = _Bwd(_ptr(x), *(w.data_ptr() for w in weights), cos.data_ptr(), sin.data_ptr(), saved.data_ptr(), res2.data_ptr(),
+                    *(g.data_ptr() for g in ctx.grads), dout.data_ptr(), _ptr(dres2), work.data_ptr(), dx.data_ptr())
+        check(lib().tsb_block_backward(shape, args, floats, int(ctx.has_res), int(causal), stream_ptr(res2.device)), "tsb_block_backward")
+        _native.add_launches(LAUNCHES_BACKWARD - 1)
+        return (dx, dx if ctx.has_res else None) + (None,) * 12
+
+
+def block_kernels_ok(x: torch.Tensor) -> bool:
+    """The settings choose the native product and attention, and the library has this file's entry points."""
+    return _use_native(x) and _native_flash_available() and hasattr(lib(), "tsb_block_forward")
+
+
+def decoder_block(x, res, weights, grads, cos, sin, shape, floats, causal):
+    """``(out, x [+ res] + attention)``; ``shape`` is (B, S, W, H, Hkv, D, F), ``floats`` both norms' eps and the softmax scale. The gradients of
+    ``weights`` are added to ``grads``."""
+    return _BlockFn.apply(x, res, *weights, grads, cos, sin, shape, floats, causal)

@@ -522,6 +522,70 @@ def test_gemm_kinds_of_tiles(dev, M, N, K, pad, a_mn, b_mn, out, accumulate):
     assert torch.equal(rows[:, N:], beside)
 
 
+def _block_model(dev, width, heads, kv, ffn, seed=0):
+    from tesseract_b200.models import LlamaConfig, LlamaModel
+    from tesseract_b200.optim import ParamArena
+    cfg = LlamaConfig(vocab_size=96, hidden_size=width, num_hidden_layers=2, num_attention_heads=heads, num_key_value_heads=kv,
+                      intermediate_size=ffn, max_position_embeddings=512, dtype=torch.bfloat16)
+    model = LlamaModel(cfg, device=dev, init_std=0.05, seed=seed)
+    return model, ParamArena.from_module(model)
+
+
+@pytest.mark.parametrize("width,heads,kv,ffn,B,S", [(128, 2, 1, 256, 1, 1), (128, 2, 2, 264, 2, 129), (256, 2, 1, 688, 3, 77), (512, 4, 4, 1032, 1, 300),
+                                                    (512, 8, 2, 1024, 2, 128)])
+def test_block_in_one_call_gives_what_its_modules_give(dev, width, heads, kv, ffn, B, S):
+    """The same launches, so the same numbers but for dQ, whose parts add up in any order, and the first block's sum of two gradients, rounded once
+    instead of twice; through two blocks each of these moves a value of bf16 by a few last bits (2^-8 each)."""
+    model, arena = _block_model(dev, width, heads, kv, ffn)
+    g = torch.Generator(device=dev).manual_seed(S)
+    tok, tgt = (torch.randint(0, 96, (B, S), device=dev, generator=g) for _ in range(2))
+    results = []
+    for hooked in (False, True):
+        handles = [blk.norm_1.register_forward_hook(lambda *a: None) for blk in model.layers] if hooked else []
+        x = model.embed_tokens(tok)
+        assert (model.layers[0]._whole(x, None) is None) is hooked
+        arena.zero_grad()
+        for _ in range(2):                                     # gradients add up
+            loss = model.loss(tok, tgt)
+            loss.backward()
+        results.append((float(loss.detach()), [p.main_grad.float().clone() for p in arena.params]))
+        for h in handles:
+            h.remove()
+    _status_ok()
+    assert results[0][0] == results[1][0]
+    for a, b in zip(results[0][1], results[1][1]):
+        assert float((a - b).norm()) <= 0.02 * float(b.norm()) + 1e-6
+
+
+def test_block_runs_its_modules_where_they_are_not_plain(dev):
+    from tesseract_b200.nn.modules import Linear
+    model, arena = _block_model(dev, 128, 2, 1, 256)
+    blk = model.layers[1]
+    x = torch.randn(2, 8, 128, device=dev, dtype=torch.bfloat16, requires_grad=True)
+    whole = lambda: blk._whole(x, None) is not None
+    assert whole()
+    for m in (blk.norm_1, blk.attn, blk.attn.v_proj, blk.norm_2, blk.ffn, blk.ffn.down_proj):
+        h = m.register_forward_pre_hook(lambda *a: None)
+        assert not whole()
+        h.remove()
+        h = m.register_full_backward_hook(lambda *a: None)
+        assert not whole()
+        h.remove()
+    blk.ffn.up_proj.weight.requires_grad_(False)
+    assert not whole()
+    blk.ffn.up_proj.weight.requires_grad_(True)
+    kept = blk.attn.k_proj
+    blk.attn.k_proj = torch.nn.Linear(128, 64, bias=False, device=dev, dtype=torch.bfloat16)
+    assert not whole()                                          # another class
+    blk.attn.k_proj = Linear(128, 64, bias=False, device=dev, dtype=torch.bfloat16)
+    assert not whole()                                          # no main_grad, apart from its neighbours
+    blk.attn.k_proj = kept
+    assert whole()
+    with torch.no_grad():
+        assert not whole()
+    assert blk._whole(x.detach(), None) is None and blk._whole(x.float(), None) is None and blk._whole(x[0], None) is None
+
+
 @pytest.mark.parametrize("H,Hkv", [(4, 2), (3, 3), (6, 2)])       # two heads of a group per CTA; two tiles of a head
 @pytest.mark.parametrize("Sq,Sk", [(1, 1), (1, 300), (127, 127), (128, 128), (129, 640), (257, 257), (300, 200)])
 @pytest.mark.parametrize("D", [64, 128])
