@@ -97,15 +97,16 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ uint32_t mx_idesc(uint32_t n, uint32_t sf_id) {
   return (sf_id << 4) | ((n >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24) | (sf_id << 29);
 }
-__device__ __forceinline__ void umma_mxf8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+__device__ __forceinline__ void umma_mxf8_if(uint32_t pred, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
                                           uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate) {
   asm volatile(
       "{\n"
-      ".reg .pred p;\n"
+      ".reg .pred p, q;\n"
       "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n"
+      "setp.ne.b32 q, %7, 0;\n"
+      "@q tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n"
       "}\n" ::"r"(tmem_d),
-      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(tmem_sfa), "r"(tmem_sfb)
+      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(tmem_sfa), "r"(tmem_sfb), "r"(pred)
       : "memory");
 }
 // This warp's 32 lanes x 4 (8) consecutive 32-bit columns: thread t writes lane (lane base + t).
@@ -323,7 +324,7 @@ gemm_decode_mx_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
   __shared__ uint32_t tmem_base_smem;
   __shared__ volatile int cta_abort;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
   const int slice = static_cast<int>(cluster_ctarank());
   const int tile = static_cast<int>(blockIdx.x) / S;
@@ -362,84 +363,88 @@ gemm_decode_mx_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      int w_issued = 0, ws = 0, x_issued = 0, xs = 0;
-      uint32_t wphase = 0, xphase = 0;
-      auto issue_w = [&]() {
+    const bool lead = elect_one();           // (the loops of warps 0 and 1 are walked by the whole warp)
+    int w_issued = 0, ws = 0, x_issued = 0, xs = 0;
+    uint32_t wphase = 0, xphase = 0;
+    auto issue_w = [&]() {
+      if (lead) {
         mbar_expect_tx(&full[ws], w_bytes);
         tma_load_2d(sW + ws * L.w_pitch, &tmW, &full[ws], (kb0 + w_issued) * BK, n0);
-        ++w_issued;
-        if (++ws == ST) {
-          ws = 0;
-          wphase ^= 1u;
-        }
-      };
-      // weights do not depend on the kernel before this one: fill the ring before waiting for it
-      while (w_issued < nk && w_issued < ST) issue_w();
-      pdl_wait();
-      long long t0 = clock64();
-      uint32_t spins = 0;
-      while (x_issued < nk || w_issued < nk) {
-        bool progress = false;
-        if (w_issued < nk && mbar_test_wait(&empty[ws], wphase ^ 1u)) {
-          issue_w();
-          progress = true;
-        }
-        if (x_issued < nk && mbar_test_wait(&empty[xs], xphase ^ 1u)) {
+      }
+      __syncwarp();
+      ++w_issued;
+      if (++ws == ST) {
+        ws = 0;
+        wphase ^= 1u;
+      }
+    };
+    // weights do not depend on the kernel before this one: fill the ring before waiting for it
+    while (w_issued < nk && w_issued < ST) issue_w();
+    pdl_wait();
+    long long t0 = clock64();
+    uint32_t spins = 0;
+    while (x_issued < nk || w_issued < nk) {
+      bool progress = false;
+      if (w_issued < nk && __all_sync(0xffffffffu, mbar_test_wait(&empty[ws], wphase ^ 1u) ? 1 : 0)) {
+        issue_w();
+        progress = true;
+      }
+      if (x_issued < nk && __all_sync(0xffffffffu, mbar_test_wait(&empty[xs], xphase ^ 1u) ? 1 : 0)) {
+        if (lead) {
           mbar_expect_tx(&full[xs], x_bytes);
 #pragma unroll
           for (int rb = 0; rb < RB; ++rb)
             tma_load_2d(sX + xs * L.x_pitch + rb * x_block, &tmX, &full[xs], (kb0 + x_issued) * BK, m0 + rb * BM);
-          ++x_issued;
-          if (++xs == ST) {
-            xs = 0;
-            xphase ^= 1u;
-          }
-          progress = true;
         }
-        if (progress) {
-          t0 = clock64();
-          spins = 0;
-        } else if ((++spins & 255u) == 0u) {
-          if (cta_abort) break;
-          if (clock64() - t0 > kWaitCycleLimit) {
-            cta_abort = 1;
-            if (status) atomicCAS(status, kStatusOk, kStatusMbarTimeout);
-            break;
-          }
+        __syncwarp();
+        ++x_issued;
+        if (++xs == ST) {
+          xs = 0;
+          xphase ^= 1u;
+        }
+        progress = true;
+      }
+      if (progress) {
+        t0 = clock64();
+        spins = 0;
+      } else if ((++spins & 255u) == 0u) {
+        if (__any_sync(0xffffffffu, cta_abort)) break;
+        if (__any_sync(0xffffffffu, clock64() - t0 > kWaitCycleLimit ? 1 : 0)) {
+          cta_abort = 1;
+          if (lead && status) atomicCAS(status, kStatusOk, kStatusMbarTimeout);
+          break;
         }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      int s = 0;
-      uint32_t phase = 0;
-      for (int i = 0; i < nk; ++i) {
-        if (!mbar_wait(&full[s], phase, &cta_abort, status)) break;
-        if (i == 0) stamp(2);                      // first stage complete (weights, activations, scales)
-        tc_fence_after();
-        const uint32_t a_base = smem_u32(sX + s * L.x_pitch);
-        const uint32_t b_base = smem_u32(sW + s * L.w_pitch);
-        const uint32_t sf_col = tmem_base + static_cast<uint32_t>(sf_base(RB) + s * kSfCols);
+    const uint32_t lead = elect_one() ? 1u : 0u;
+    int s = 0;
+    uint32_t phase = 0;
+    for (int i = 0; i < nk; ++i) {
+      if (!mbar_wait_warp(&full[s], phase, &cta_abort, status)) break;
+      if (lead && i == 0) stamp(2);                      // first stage complete (weights, activations, scales)
+      tc_fence_after();
+      const uint32_t a_base = smem_u32(sX + s * L.x_pitch);
+      const uint32_t b_base = smem_u32(sW + s * L.w_pitch);
+      const uint32_t sf_col = tmem_base + static_cast<uint32_t>(sf_base(RB) + s * kSfCols);
 #pragma unroll
-        for (int rb = 0; rb < RB; ++rb) {
+      for (int rb = 0; rb < RB; ++rb) {
 #pragma unroll
-          for (int k = 0; k < BK / 32; ++k)
-            umma_mxf8(tmem_base + static_cast<uint32_t>(rb * d_stride(RB)),
-                      umma_smem_desc_sw128(a_base + rb * x_block + k * 32, 16, 1024),
-                      umma_smem_desc_sw128(b_base + k * 32, 16, 1024), mx_idesc(static_cast<uint32_t>(BN), k),
-                      sf_col + static_cast<uint32_t>(rb * 4), sf_col + 8u, (i | k) != 0 ? 1u : 0u);
-        }
-        umma_commit(&empty[s]);
-        if (++s == ST) {
-          s = 0;
-          phase ^= 1u;
-        }
+        for (int k = 0; k < BK / 32; ++k)
+          umma_mxf8_if(lead, tmem_base + static_cast<uint32_t>(rb * d_stride(RB)),
+                    umma_smem_desc_sw128(a_base + rb * x_block + k * 32, 16, 1024),
+                    umma_smem_desc_sw128(b_base + k * 32, 16, 1024), mx_idesc(static_cast<uint32_t>(BN), k),
+                    sf_col + static_cast<uint32_t>(rb * 4), sf_col + 8u, (i | k) != 0 ? 1u : 0u);
       }
-      umma_commit(&acc_bar);
-      stamp(3);                                    // last MMA issued
+      umma_commit_if(lead, &empty[s]);
+      if (++s == ST) {
+        s = 0;
+        phase ^= 1u;
+      }
     }
+    umma_commit_if(lead, &acc_bar);
+    if (lead) stamp(3);                                    // last MMA issued
   } else {
     // ------------------------------------------------------------ scale warps (2 .. 5): one lane quadrant each
     const int q = warp & 3;

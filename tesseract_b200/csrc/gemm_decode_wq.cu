@@ -20,6 +20,9 @@
 //     predecessor) happen before griddepcontrol.wait; only the activation loads come after it. In a decode step,
 //     where a GEMM lasts 5 to 40 microseconds, this hides the launch ramp behind the previous kernel's tail.
 // Accumulation: tcgen05.mma kind::f16, 128 x BN x 16, fp32 in TMEM. All waits are bounded (common.cuh).
+// A step of K costs four MMAs and the loop that issues them, which the whole warp walks (elect_one); one lane's loop took longer than the bytes of
+// a step. Launches behind one another, us, one lane -> warp, [N, K] at 64 rows: 6144 x 4096 16.1 -> 14.5, 4096 x 4096 14.7 -> 12.8,
+// 4096 x 14336 34.0 -> 27.1 (4.3 TB/s), 28672 x 4096 41.4 -> 41.0 (5.7 TB/s), 1024 x 1024 7.0 -> 5.8.
 //
 // Replaces the reference's cuBLASLt call for M <= 16 .. 256 (src/cuda/MatMul.cpp:422-490) and its dequantising
 // CUDA-core kernels for quantised weights at batch sizes above a GEMV (src/cuda/DequantMatMul.cu:95-127).
@@ -159,7 +162,7 @@ gemm_decode_wq_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
   __shared__ uint32_t tmem_base_smem;
   __shared__ volatile int cta_abort;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
   const int slice = static_cast<int>(cluster_ctarank());
   const int tile = static_cast<int>(blockIdx.x) / S;
@@ -209,18 +212,19 @@ gemm_decode_wq_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      const int WST = FP8 ? L.r_stages : L.c_stages;
-      const bool packed = (flags & 2) != 0;
-      const uint32_t x_bytes = static_cast<uint32_t>(RB * L.x_rows) * BK * 2;
-      uint64_t* w_full = FP8 ? full_r : full_c;
-      uint64_t* w_empty = FP8 ? empty_r : empty_c;
-      uint8_t* w_base = FP8 ? sR : sC;
-      const int x_row = m0 + x_off;
-      const uint32_t w_pitch = static_cast<uint32_t>(FP8 ? L.r_pitch : L.c_pitch);
-      int w_issued = 0, ws = 0, x_issued = 0, xs = 0;
-      uint32_t wphase = 0, xphase = 0;
-      auto issue_w = [&]() {
+    const bool lead = elect_one();           // (the loops of warps 0 and 1 are walked by the whole warp)
+    const int WST = FP8 ? L.r_stages : L.c_stages;
+    const bool packed = (flags & 2) != 0;
+    const uint32_t x_bytes = static_cast<uint32_t>(RB * L.x_rows) * BK * 2;
+    uint64_t* w_full = FP8 ? full_r : full_c;
+    uint64_t* w_empty = FP8 ? empty_r : empty_c;
+    uint8_t* w_base = FP8 ? sR : sC;
+    const int x_row = m0 + x_off;
+    const uint32_t w_pitch = static_cast<uint32_t>(FP8 ? L.r_pitch : L.c_pitch);
+    int w_issued = 0, ws = 0, x_issued = 0, xs = 0;
+    uint32_t wphase = 0, xphase = 0;
+    auto issue_w = [&]() {
+      if (lead) {
         mbar_expect_tx(&w_full[ws], w_stage_bytes);
         if (packed)   // tile-major weights: tile (n tile, k step) is one contiguous run of BN * 64 bytes
           bulk_load(w_base + ws * w_pitch,
@@ -228,88 +232,94 @@ gemm_decode_wq_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
                     &w_full[ws]);
         else
           tma_load_2d(w_base + ws * w_pitch, &tmW, &w_full[ws], (kb0 + w_issued) * BK, n0);
-        ++w_issued;
-        if (++ws == WST) {
-          ws = 0;
-          wphase ^= 1u;
-        }
-      };
-      // weights do not depend on the kernel before this one: fill the ring before waiting for it
-      while (w_issued < nk && w_issued < WST) issue_w();
-      pdl_wait();
-      // The two rings advance independently: whichever has a free slot gets its next load, so the (small)
-      // activation loads never queue behind a weight slot that is still being multiplied.
-      long long t0 = clock64();
-      uint32_t spins = 0;
-      while (x_issued < nk || w_issued < nk) {
-        bool progress = false;
-        if (w_issued < nk && mbar_test_wait(&w_empty[ws], wphase ^ 1u)) {
-          issue_w();
-          progress = true;
-        }
-        if (x_issued < nk && mbar_test_wait(&empty_x[xs], xphase ^ 1u)) {
+      }
+      __syncwarp();
+      ++w_issued;
+      if (++ws == WST) {
+        ws = 0;
+        wphase ^= 1u;
+      }
+    };
+    // weights do not depend on the kernel before this one: fill the ring before waiting for it
+    while (w_issued < nk && w_issued < WST) issue_w();
+    pdl_wait();
+    // The two rings advance independently: whichever has a free slot gets its next load, so the (small)
+    // activation loads never queue behind a weight slot that is still being multiplied.
+    long long t0 = clock64();
+    uint32_t spins = 0;
+    while (x_issued < nk || w_issued < nk) {
+      bool progress = false;
+      if (w_issued < nk && __all_sync(0xffffffffu, mbar_test_wait(&w_empty[ws], wphase ^ 1u) ? 1 : 0)) {
+        issue_w();
+        progress = true;
+      }
+      if (x_issued < nk && __all_sync(0xffffffffu, mbar_test_wait(&empty_x[xs], xphase ^ 1u) ? 1 : 0)) {
+        if (lead) {
           mbar_expect_tx(&full_x[xs], x_bytes);
 #pragma unroll
           for (int rb = 0; rb < RB; ++rb)
             tma_load_2d(sX + xs * L.x_pitch + rb * kXBlock, &tmX, &full_x[xs], (kb0 + x_issued) * BK, x_row + rb * BM);
-          ++x_issued;
-          if (++xs == L.x_stages) {
-            xs = 0;
-            xphase ^= 1u;
-          }
-          progress = true;
         }
-        if (progress) {
-          t0 = clock64();
-          spins = 0;
-        } else if ((++spins & 255u) == 0u) {
-          if (cta_abort) break;
-          if (clock64() - t0 > kWaitCycleLimit) {
-            cta_abort = 1;
-            if (status) atomicCAS(status, kStatusOk, kStatusMbarTimeout);
-            break;
-          }
+        __syncwarp();
+        ++x_issued;
+        if (++xs == L.x_stages) {
+          xs = 0;
+          xphase ^= 1u;
+        }
+        progress = true;
+      }
+      if (progress) {
+        t0 = clock64();
+        spins = 0;
+      } else if ((++spins & 255u) == 0u) {
+        if (__any_sync(0xffffffffu, cta_abort)) break;
+        if (__any_sync(0xffffffffu, clock64() - t0 > kWaitCycleLimit ? 1 : 0)) {
+          cta_abort = 1;
+          if (lead && status) atomicCAS(status, kStatusOk, kStatusMbarTimeout);
+          break;
         }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc(BM, static_cast<uint32_t>(BN), 1, 1, 0, 0);   // bf16 x bf16 -> fp32
-      int xs = 0, cs = 0;
-      uint32_t xphase = 0, cphase = 0;
-      for (int i = 0; i < nk; ++i) {
-        if (!mbar_wait(&full_x[xs], xphase, &cta_abort, status)) break;
-        if (!mbar_wait(&full_c[cs], cphase, &cta_abort, status)) break;
-        tc_fence_after();
-        const uint32_t a_base = smem_u32(sX + xs * L.x_pitch);
-        const uint32_t b_base = smem_u32(sC + cs * L.c_pitch);
-        if (flags & 1) {        // measurement aid: consume the stages without multiplying
+    const uint32_t lead = elect_one() ? 1u : 0u;
+    const uint32_t idesc = umma_idesc(BM, static_cast<uint32_t>(BN), 1, 1, 0, 0);   // bf16 x bf16 -> fp32
+    int xs = 0, cs = 0;
+    uint32_t xphase = 0, cphase = 0;
+    for (int i = 0; i < nk; ++i) {
+      if (!mbar_wait_warp(&full_x[xs], xphase, &cta_abort, status)) break;
+      if (!mbar_wait_warp(&full_c[cs], cphase, &cta_abort, status)) break;
+      tc_fence_after();
+      const uint32_t a_base = smem_u32(sX + xs * L.x_pitch);
+      const uint32_t b_base = smem_u32(sC + cs * L.c_pitch);
+      if (flags & 1) {        // measurement aid: consume the stages without multiplying
+        if (lead) {
           mbar_arrive(&empty_x[xs]);
           mbar_arrive(&empty_c[cs]);
-        } else {
+        }
+        __syncwarp();
+      } else {
 #pragma unroll
-          for (int rb = 0; rb < RB; ++rb) {
+        for (int rb = 0; rb < RB; ++rb) {
 #pragma unroll
-            for (int k = 0; k < BK / 16; ++k)
-              umma_f16(tmem_base + static_cast<uint32_t>(rb * kMaxBN),
-                       umma_smem_desc_sw128(a_base + rb * kXBlock + k * 32, 16, 1024),
-                       umma_smem_desc_sw128(b_base + k * 32, 16, 1024), idesc, (i | k) != 0 ? 1u : 0u);
-          }
-          umma_commit(&empty_x[xs]);
-          umma_commit(&empty_c[cs]);
+          for (int k = 0; k < BK / 16; ++k)
+            umma_f16_if(lead, tmem_base + static_cast<uint32_t>(rb * kMaxBN),
+                     umma_smem_desc_sw128(a_base + rb * kXBlock + k * 32, 16, 1024),
+                     umma_smem_desc_sw128(b_base + k * 32, 16, 1024), idesc, (i | k) != 0 ? 1u : 0u);
         }
-        if (++xs == L.x_stages) {
-          xs = 0;
-          xphase ^= 1u;
-        }
-        if (++cs == CST) {
-          cs = 0;
-          cphase ^= 1u;
-        }
+        umma_commit_if(lead, &empty_x[xs]);
+        umma_commit_if(lead, &empty_c[cs]);
       }
-      umma_commit(&acc_bar);
+      if (++xs == L.x_stages) {
+        xs = 0;
+        xphase ^= 1u;
+      }
+      if (++cs == CST) {
+        cs = 0;
+        cphase ^= 1u;
+      }
     }
+    umma_commit_if(lead, &acc_bar);
   } else if (warp >= 6) {
     // ------------------------------------------------------------ fp8 -> bf16 conversion warps
     if (FP8) {

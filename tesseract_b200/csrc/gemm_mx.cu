@@ -23,6 +23,9 @@
 // A first version wrote the scales into tensor memory from four extra warps with tcgen05.st behind the stage barriers;
 // it was correct and ran at 1100 TFLOP/s (8192^3), below the bf16 GEMM: every stage paid a cross-warp round trip.
 //
+// The loops of warps 0 and 1 are walked by the whole warp (elect_one). L2 flushed before each launch, one lane's loop -> warp's loop, TFLOP/s:
+// 8192^3 2020 -> 2758, 16384 x 4096 x 4096 1864 -> 2494, 16384 x 28672 x 4096 2047 -> 2481, 16384 x 4096 x 14336 1991 -> 2745.
+//
 // The reference's fp8 GEMM is one scale per tensor through cuBLASLt (src/cuda/Fp8MatMul.cu:93-157).
 #include "common.cuh"
 
@@ -61,15 +64,16 @@ __device__ __forceinline__ Tile tile_of(int t, int num_m, int num_n) {
 __device__ __forceinline__ uint32_t mx_idesc(uint32_t n, uint32_t sf_id) {
   return (sf_id << 4) | ((n >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24) | (sf_id << 29);
 }
-__device__ __forceinline__ void umma_mxf8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+__device__ __forceinline__ void umma_mxf8_if(uint32_t pred, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
                                           uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate) {
   asm volatile(
       "{\n"
-      ".reg .pred p;\n"
+      ".reg .pred p, q;\n"
       "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n"
+      "setp.ne.b32 q, %7, 0;\n"
+      "@q tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n"
       "}\n" ::"r"(tmem_d),
-      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(tmem_sfa), "r"(tmem_sfb)
+      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(tmem_sfa), "r"(tmem_sfb), "r"(pred)
       : "memory");
 }
 // Shared-memory descriptor of one scale atom for tcgen05.cp: 32 rows of 16 bytes, K-major, no swizzle; 8-row core
@@ -81,8 +85,15 @@ __device__ __forceinline__ uint64_t sf_smem_desc(uint32_t smem_addr) {
   d |= static_cast<uint64_t>(1) << 46;  // descriptor version for sm_100
   return d;
 }
-__device__ __forceinline__ void tmem_cp_32x128b_x4(uint32_t taddr, uint64_t sdesc) {
-  asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
+__device__ __forceinline__ void tmem_cp_32x128b_x4_if(uint32_t pred, uint32_t taddr, uint64_t sdesc) {
+  asm volatile(
+      "{\n"
+      ".reg .pred q;\n"
+      "setp.ne.b32 q, %2, 0;\n"
+      "@q tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n"
+      "}\n" ::"r"(taddr),
+      "l"(sdesc), "r"(pred)
+      : "memory");
 }
 
 __global__ void __launch_bounds__(kThreads, 1)
@@ -96,7 +107,7 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   __shared__ uint32_t tmem_base_smem;
   __shared__ volatile int cta_abort;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
   const int num_m = (M + BM - 1) / BM;
   const int num_n = (N + BN - 1) / BN;
@@ -129,78 +140,79 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        const Tile tc = tile_of(t, num_m, num_n);
-        const int m0 = tc.m_blk * BM, n0 = tc.n_blk * BN;
-        const int atom0 = n0 >> 7;                               // weight atom that holds the tile's first row
-        const int atom1 = min(atom0 + 1, n_atoms - 1);
-        for (int kb = 0; kb < nkb; ++kb) {
-          ok = mbar_wait(&empty_bar[stage], phase ^ 1u, &cta_abort, status);
-          if (!ok) break;
-          uint8_t* sA = smem + stage * kStage;
-          uint8_t* sB = sA + kStageA;
-          uint8_t* sS = sB + kStageB;
+    const bool lead = elect_one();           // (the loops of warps 0 and 1 are walked by the whole warp)
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      const Tile tc = tile_of(t, num_m, num_n);
+      const int m0 = tc.m_blk * BM, n0 = tc.n_blk * BN;
+      const int atom0 = n0 >> 7;                               // weight atom that holds the tile's first row
+      const int atom1 = min(atom0 + 1, n_atoms - 1);
+      for (int kb = 0; kb < nkb; ++kb) {
+        ok = mbar_wait_warp(&empty_bar[stage], phase ^ 1u, &cta_abort, status);
+        if (!ok) break;
+        uint8_t* sA = smem + stage * kStage;
+        uint8_t* sB = sA + kStageA;
+        uint8_t* sS = sB + kStageB;
+        if (lead) {
           mbar_expect_tx(&full_bar[stage], static_cast<uint32_t>(kStageA + kStageB + kStageSf));
           tma_load_2d(sA, &tmA, &full_bar[stage], kb * BK, m0);
           tma_load_2d(sB, &tmB, &full_bar[stage], kb * BK, n0);
           bulk_load(sS, sfa + (static_cast<long long>(tc.m_blk) * nkb + kb) * kAtom, kAtom, &full_bar[stage]);
           bulk_load(sS + kAtom, sfb + (static_cast<long long>(atom0) * nkb + kb) * kAtom, kAtom, &full_bar[stage]);
           bulk_load(sS + 2 * kAtom, sfb + (static_cast<long long>(atom1) * nkb + kb) * kAtom, kAtom, &full_bar[stage]);
-          if (++stage == kStages) {
-            stage = 0;
-            phase ^= 1u;
-          }
+        }
+        __syncwarp();
+        if (++stage == kStages) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      int acc = 0;
-      uint32_t acc_phase = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        const Tile tc = tile_of(t, num_m, num_n);
-        const int n0 = tc.n_blk * BN;
-        ok = mbar_wait(&tmem_empty_bar[acc], acc_phase ^ 1u, &cta_abort, status);
+    const uint32_t lead = elect_one() ? 1u : 0u;
+    int stage = 0;
+    uint32_t phase = 0;
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      const Tile tc = tile_of(t, num_m, num_n);
+      const int n0 = tc.n_blk * BN;
+      ok = mbar_wait_warp(&tmem_empty_bar[acc], acc_phase ^ 1u, &cta_abort, status);
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
+      const uint32_t sfa_t = tmem_base + kSfaCol;
+      const uint32_t sfb_t = tmem_base + kSfbCol;
+      const uint32_t sfb_read = sfb_t + static_cast<uint32_t>((n0 & 127) >> 5);   // 0 or 2: the tile starts 0 / 64 rows in
+      for (int kb = 0; kb < nkb; ++kb) {
+        ok = mbar_wait_warp(&full_bar[stage], phase, &cta_abort, status);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
-        const uint32_t sfa_t = tmem_base + kSfaCol;
-        const uint32_t sfb_t = tmem_base + kSfbCol;
-        const uint32_t sfb_read = sfb_t + static_cast<uint32_t>((n0 & 127) >> 5);   // 0 or 2: the tile starts 0 / 64 rows in
-        for (int kb = 0; kb < nkb; ++kb) {
-          ok = mbar_wait(&full_bar[stage], phase, &cta_abort, status);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t a_base = smem_u32(smem + stage * kStage);
-          const uint32_t b_base = a_base + kStageA;
-          const uint32_t s_base = b_base + kStageB;
-          tmem_cp_32x128b_x4(sfa_t, sf_smem_desc(s_base));
-          tmem_cp_32x128b_x4(sfb_t, sf_smem_desc(s_base + kAtom));
-          tmem_cp_32x128b_x4(sfb_t + 4, sf_smem_desc(s_base + 2 * kAtom));
+        const uint32_t a_base = smem_u32(smem + stage * kStage);
+        const uint32_t b_base = a_base + kStageA;
+        const uint32_t s_base = b_base + kStageB;
+        tmem_cp_32x128b_x4_if(lead, sfa_t, sf_smem_desc(s_base));
+        tmem_cp_32x128b_x4_if(lead, sfb_t, sf_smem_desc(s_base + kAtom));
+        tmem_cp_32x128b_x4_if(lead, sfb_t + 4, sf_smem_desc(s_base + 2 * kAtom));
 #pragma unroll
-          for (int k = 0; k < BK / 32; ++k)
-            umma_mxf8(d_tmem, umma_smem_desc_sw128(a_base + k * 32, 16, 1024),
-                      umma_smem_desc_sw128(b_base + k * 32, 16, 1024), mx_idesc(BN, k), sfa_t, sfb_read,
-                      (kb | k) != 0 ? 1u : 0u);
-          umma_commit(&empty_bar[stage]);
-          if (++stage == kStages) {
-            stage = 0;
-            phase ^= 1u;
-          }
+        for (int k = 0; k < BK / 32; ++k)
+          umma_mxf8_if(lead, d_tmem, umma_smem_desc_sw128(a_base + k * 32, 16, 1024),
+                    umma_smem_desc_sw128(b_base + k * 32, 16, 1024), mx_idesc(BN, k), sfa_t, sfb_read,
+                    (kb | k) != 0 ? 1u : 0u);
+        umma_commit_if(lead, &empty_bar[stage]);
+        if (++stage == kStages) {
+          stage = 0;
+          phase ^= 1u;
         }
-        if (!ok) break;
-        umma_commit(&tmem_full_bar[acc]);
-        acc ^= 1;
-        if (acc == 0) acc_phase ^= 1u;
       }
+      if (!ok) break;
+      umma_commit_if(lead, &tmem_full_bar[acc]);
+      acc ^= 1;
+      if (acc == 0) acc_phase ^= 1u;
     }
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..5)
