@@ -3,7 +3,7 @@
 //
 // What bounds a training step of a small model is the host: a block is 9 launches forward and 20 backward, and issuing each through Python,
 // autograd and ctypes took 29 us of host time, where the GPU worked 2 - 10 (4 layers of width 256, 4 x 128 tokens: 4.2 ms a step, 0.65 of them
-// kernels). BLOCKFIGS
+// kernels). From here: 1.53 ms.
 #include "common.cuh"
 
 TSB_EXPORT int tsb_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* h_out, float* rstd, int rows, int D, float eps,

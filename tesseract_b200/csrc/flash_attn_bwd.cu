@@ -58,7 +58,7 @@ struct BwdCfg {
   static constexpr int kPieces = D == 64 ? 3 : 0, kPieceBytes = 32 * 16 * 4;   // a warp's ring of pieces of dQ, 32 rows x 16 columns
   static constexpr int kSmemBytes =
       (2 + kQStages + kDOStages) * kTileBytes + BT * BT * 2 + kQStages * kRowBytes + 4 * kPieces * kPieceBytes + 1024;
-  // heads of 64 leave room for dQ; with 128 columns it lies over dP
+  static constexpr bool kOwnDQ = D == 64;           // heads of 64 leave room for dQ; with 128 columns it lies over dP
   static constexpr int kColS = 0, kColDP = 128, kColDV = 256, kColDK = 256 + D, kColDQ = D == 128 ? kColDP : 384;
 };
 
@@ -222,37 +222,49 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           umma_commit_if(lead, &s_full);
           return true;
         };
-        bool ok = mbar_wait_warp(&kv_full, 0, &cta_abort, p.status) && scores(0);
+        auto gradients_of_p = [&](int t) -> bool {     // dP^T = V dO^T
+          const int ds = t % Cfg::kDOStages;
+          if (!mbar_wait_warp(&do_full[ds], (t / Cfg::kDOStages) & 1, &cta_abort, p.status)) return false;
+          // (with 128 columns dQ of the step before lies here)
+          if (!Cfg::kOwnDQ && !mbar_wait_warp(&dq_read, (t & 1) ^ 1u, &cta_abort, p.status)) return false;
+          tc_fence_after();
+          const uint32_t do_base = smem_u32(sDO + ds * Cfg::kTileBytes);
+#pragma unroll
+          for (int ks = 0; ks < D / 16; ++ks)
+            umma_f16_if(lead, tmem_base + Cfg::kColDP, kmajor_desc<128>(v_base, ks), kmajor_desc<128>(do_base, ks), idesc_s, ks != 0);
+          umma_commit_if(lead, &dp_full);
+          return true;
+        };
+        bool ok = mbar_wait_warp(&kv_full, 0, &cta_abort, p.status) && scores(0) && (!Cfg::kOwnDQ || gradients_of_p(0));
         for (int t = 0; ok && t < n_iter; ++t) {
           const uint32_t ph = t & 1;
           const uint32_t q_base = smem_u32(sQ + (t % Cfg::kQStages) * Cfg::kTileBytes);
           const uint32_t do_base = smem_u32(sDO + (t % Cfg::kDOStages) * Cfg::kTileBytes);
-          if (!mbar_wait_warp(&do_full[t % Cfg::kDOStages], (t / Cfg::kDOStages) & 1, &cta_abort, p.status)) break;
-          if (!mbar_wait_warp(&dq_read, ph ^ 1u, &cta_abort, p.status)) break;
-          tc_fence_after();
-#pragma unroll
-          for (int ks = 0; ks < D / 16; ++ks)    // dP^T = V dO^T
-            umma_f16_if(lead, tmem_base + Cfg::kColDP, kmajor_desc<128>(v_base, ks), kmajor_desc<128>(do_base, ks), idesc_s, ks != 0);
-          umma_commit_if(lead, &dp_full);
+          if (!Cfg::kOwnDQ && !gradients_of_p(t)) break;
           if (!mbar_wait_warp(&p_full, ph, &cta_abort, p.status)) break;
           tc_fence_after();
 #pragma unroll
           for (int ks = 0; ks < BT / 16; ++ks)   // dV += P^T dO   (K = query rows; each half of P^T lies over its half of S^T)
-            umma_f16_ts_if(lead, tmem_base + Cfg::kColDV, tmem_base + Cfg::kColS + (ks >> 2) * 64 + (ks & 3) * 8, mnmajor_desc(do_base, ks, 16384),
-                        idesc_kv, (t | ks) != 0);
+            umma_f16_ts_if(lead, tmem_base + Cfg::kColDV, tmem_base + Cfg::kColS + (ks >> 2) * 64 + (ks & 3) * 8,
+                           mnmajor_desc(do_base, ks, 16384), idesc_kv, (t | ks) != 0);
           umma_commit_if(lead, &do_empty[t % Cfg::kDOStages]);
           if (t + 1 < n_iter && !scores(t + 1)) break;
           if (!mbar_wait_warp(&ds_full, ph, &cta_abort, p.status)) break;
           tc_fence_after();
 #pragma unroll
           for (int ks = 0; ks < BT / 16; ++ks)   // dK += dS^T Q
-            umma_f16_ts_if(lead, tmem_base + Cfg::kColDK, tmem_base + Cfg::kColDP + (ks >> 2) * 64 + (ks & 3) * 8, mnmajor_desc(q_base, ks, 16384),
-                        idesc_kv, (t | ks) != 0);
+            umma_f16_ts_if(lead, tmem_base + Cfg::kColDK, tmem_base + Cfg::kColDP + (ks >> 2) * 64 + (ks & 3) * 8,
+                           mnmajor_desc(q_base, ks, 16384), idesc_kv, (t | ks) != 0);
+          umma_commit_if(lead, &q_empty[t % Cfg::kQStages]);
+          if (Cfg::kOwnDQ) {
+            if (t + 1 < n_iter && !gradients_of_p(t + 1)) break;
+            if (!mbar_wait_warp(&dq_read, ph ^ 1u, &cta_abort, p.status)) break;
+            tc_fence_after();
+          }
 #pragma unroll
           for (int ks = 0; ks < BT / 16; ++ks)   // dQ = dS K       (K = key rows; with 128 columns over dS^T, which dK has read)
             umma_f16_if(lead, tmem_base + Cfg::kColDQ, mnmajor_desc(ds_base, ks, 16384), mnmajor_desc(k_base, ks, 16384), idesc_q, ks != 0);
           umma_commit_if(lead, &dq_full);
-          umma_commit_if(lead, &q_empty[t % Cfg::kQStages]);
         }
       }
     }
