@@ -42,6 +42,7 @@ _SIGNATURES = {
     "tsb_adam_flat": [P, P, P, P, P, L, F, F, F, F, F, F, F, P, I, I, P],
     "tsb_adam_chunk_elems": [],
     "tsb_adam_multi": [P, P, I, F, F, F, F, F, F, F, P, I, I, P],
+    "tsb_zero": [P, L, P],
     "tsb_sumsq": [P, L, P, I, P],
     "tsb_clip_coef": [P, P, F, F, P],
 }

@@ -367,6 +367,24 @@ __device__ __forceinline__ int mx_exponent_byte(float amax) {
 }
 __device__ __forceinline__ float mx_inv_scale(int e) { return __uint_as_float(static_cast<uint32_t>(254 - e) << 23); }
 
+// ---------------------------------------------------------------- 32 bytes at once (aligned to them)
+struct Bytes32 {
+  uint32_t w[8];
+};
+__device__ __forceinline__ Bytes32 ld_global_32(const void* p) {
+  Bytes32 v;
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v.w[0]), "=r"(v.w[1]), "=r"(v.w[2]), "=r"(v.w[3]), "=r"(v.w[4]), "=r"(v.w[5]), "=r"(v.w[6]), "=r"(v.w[7])
+               : "l"(p)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_global_32(void* p, const Bytes32& v) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v.w[0]), "r"(v.w[1]), "r"(v.w[2]), "r"(v.w[3]),
+               "r"(v.w[4]), "r"(v.w[5]), "r"(v.w[6]), "r"(v.w[7])
+               : "memory");
+}
+
 // ---------------------------------------------------------------- small math helpers
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll

@@ -14,6 +14,8 @@ from typing import Iterable
 import torch
 from torch import nn
 
+from .._native import check, lib, stream_ptr
+
 _ALIGN_ELEMS = 128  # every parameter starts on a 256-byte (bf16) / 512-byte (fp32) boundary
 
 
@@ -62,8 +64,16 @@ class ParamArena:
                 params.append(p)
         return cls(params, **kw)
 
+    def _zero(self) -> None:
+        g = self.grad
+        size = g.numel() * g.element_size()
+        if g.is_cuda and size % 32 == 0 and g.data_ptr() % 32 == 0 and hasattr(lib(), "tsb_zero"):
+            check(lib().tsb_zero(g.data_ptr(), size, stream_ptr(g.device)), "tsb_zero")
+        else:
+            g.zero_()
+
     def zero_grad(self) -> None:
-        self.grad.zero_()
+        self._zero()
         for p in self.params:
             p.grad = None
 

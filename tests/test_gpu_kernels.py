@@ -586,6 +586,37 @@ def test_block_runs_its_modules_where_they_are_not_plain(dev):
     assert blk._whole(x.detach(), None) is None and blk._whole(x.float(), None) is None and blk._whole(x[0], None) is None
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,F,shift", [(1, 16, 0), (3, 2048, 0), (5, 2064, 0), (700, 4112, 0), (66000, 16, 0), (7, 2056, 0), (9, 2048, 8)])
+def test_swiglu_in_pieces_of_32_bytes(dev, dtype, rows, F, shift):
+    """Edges of the wide kernels (last CTA of a row, second row of a thread, more rows than the grid), and what keeps the others: F off 16, rows off 32
+    bytes. Values of a few units: one rounding of the type's precision each, plus fp32 exponentials (2^-20)."""
+    from tesseract_b200 import _native
+    g = torch.Generator(device=dev).manual_seed(F)
+    def t(n):
+        return torch.randn(n + shift, device=dev, generator=g).to(dtype)[shift:]
+    gu, do = t(rows * 2 * F).view(rows, 2 * F), t(rows * F).view(rows, F)
+    out, dgu = t(rows * F).view(rows, F), t(rows * 2 * F).view(rows, 2 * F)
+    code, s = _native.dtype_code(dtype), _native.stream_ptr(dev)
+    _native.check(_native.lib().tsb_swiglu_fwd(gu.data_ptr(), out.data_ptr(), rows, F, code, s), "fwd")
+    _native.check(_native.lib().tsb_swiglu_bwd(do.data_ptr(), gu.data_ptr(), dgu.data_ptr(), rows, F, code, s), "bwd")
+    x = gu.double().requires_grad_()
+    ref = torch.nn.functional.silu(x[:, :F]) * x[:, F:]
+    ref.backward(do.double())
+    eps = torch.finfo(dtype).eps / 2 + 2.0 ** -18
+    assert bool(((out.double() - ref).abs() <= ref.abs() * eps + 1e-6).all())
+    assert bool(((dgu.double() - x.grad).abs() <= x.grad.abs() * eps + 2e-6).all())
+
+
+@pytest.mark.parametrize("size", [32, 4096, 148 * 32 * 256 * 32 + 32, 1 << 30])
+def test_zeroes(dev, size):
+    from tesseract_b200 import _native
+    x = torch.full((size + 64,), 7, dtype=torch.uint8, device=dev)
+    _native.check(_native.lib().tsb_zero(x[32:].data_ptr(), size, _native.stream_ptr(x.device)), "tsb_zero")
+    assert int(x[:32].min()) == 7 and int(x[32 + size:].min()) == 7 and int(x[32:32 + size].max()) == 0
+    assert _native.lib().tsb_zero(x[16:].data_ptr(), 32, 0) == -2 and _native.lib().tsb_zero(x.data_ptr(), 33, 0) == -2
+
+
 @pytest.mark.parametrize("H,Hkv", [(4, 2), (3, 3), (6, 2)])       # two heads of a group per CTA; two tiles of a head
 @pytest.mark.parametrize("Sq,Sk", [(1, 1), (1, 300), (127, 127), (128, 128), (129, 640), (257, 257), (300, 200)])
 @pytest.mark.parametrize("D", [64, 128])
