@@ -22,6 +22,7 @@ P, I, L, F = _native.P, _native.I, _native.L, _native.F
 _native.register_signatures({
     "tsb_paged_decode": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, F, I, I, P],
     "tsb_paged_decode_mx": [P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, F, I, I, P],
+    "tsb_rope_append_paged": [P, P, P, P, P, P, P, I, I, I, I, I, I, P],
     "tsb_paged_decode_scratch_floats": [I, I, I, I],
     "tsb_paged_decode_static_need_floats": [I, I, I, I, I, I],
     "tsb_kv_append_paged": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P],

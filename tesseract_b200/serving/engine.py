@@ -293,13 +293,18 @@ class ServingEngine(EngineCore):
                                                max_len_hint=self.cfg.max_seq_len)
                 o = o.view(T, H * D)
         else:
-            qkv = ops.rope_qkv(qkv, rope.cos, rope.sin, num_heads=H, num_kv_heads=Hkv, head_dim=D, seq_len=1,
-                               positions=positions)
-            check(lib().tsb_kv_append_paged(qkv.data_ptr(), rope.cos.data_ptr(), rope.sin.data_ptr(), positions.data_ptr(),
-                                            slots.data_ptr(), self.k_pool[li].data_ptr(), self.v_pool[li].data_ptr(),
-                                            ks.data_ptr() if ks is not None else None,
-                                            vs.data_ptr() if vs is not None else None, None, T, H, Hkv, D,
-                                            self.cfg.block_size, dt, 0, stream_ptr(qkv.device)), "tsb_kv_append_paged")
+            if ks is None and D in (64, 128) and hasattr(lib(), "tsb_rope_append_paged"):
+                check(lib().tsb_rope_append_paged(qkv.data_ptr(), rope.cos.data_ptr(), rope.sin.data_ptr(), positions.data_ptr(), slots.data_ptr(),
+                                                  self.k_pool[li].data_ptr(), self.v_pool[li].data_ptr(), T, H, Hkv, D, self.cfg.block_size, dt,
+                                                  stream_ptr(qkv.device)), "tsb_rope_append_paged")
+            else:
+                qkv = ops.rope_qkv(qkv, rope.cos, rope.sin, num_heads=H, num_kv_heads=Hkv, head_dim=D, seq_len=1,
+                                   positions=positions)
+                check(lib().tsb_kv_append_paged(qkv.data_ptr(), rope.cos.data_ptr(), rope.sin.data_ptr(), positions.data_ptr(),
+                                                slots.data_ptr(), self.k_pool[li].data_ptr(), self.v_pool[li].data_ptr(),
+                                                ks.data_ptr() if ks is not None else None,
+                                                vs.data_ptr() if vs is not None else None, None, T, H, Hkv, D,
+                                                self.cfg.block_size, dt, 0, stream_ptr(qkv.device)), "tsb_kv_append_paged")
             cu, max_len, spans = prefill_bounds
             q4 = qkv.view(T, H + 2 * Hkv, D)
             if self.varlen_prefill:

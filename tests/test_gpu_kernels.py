@@ -608,6 +608,38 @@ def test_swiglu_in_pieces_of_32_bytes(dev, dtype, rows, F, shift):
     assert bool(((dgu.double() - x.grad).abs() <= x.grad.abs() * eps + 2e-6).all())
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("tokens,H,Hkv,D,bs", [(1, 4, 2, 64, 8), (77, 3, 3, 128, 16), (2051, 32, 8, 128, 16), (700, 5, 1, 64, 12)])
+def test_prompt_rotation_and_append_in_one_pass(dev, dtype, tokens, H, Hkv, D, bs):
+    """Against the two kernels that it stands for: values the same bits; rotated ones may round x c - y s once more or less in fp32 (the compiler
+    fuses either product), 2^-23 of the terms, which can move the last bit of a stored value; a token without a slot is not stored."""
+    from tesseract_b200 import _native, ops
+    g = torch.Generator(device=dev).manual_seed(tokens)
+    nb = tokens // bs + 2
+    qkv = torch.randn(tokens, (H + 2 * Hkv) * D, device=dev, generator=g).to(dtype)
+    pools = [torch.randn(nb, Hkv, bs, D, device=dev, generator=g).to(dtype) for _ in range(2)]
+    cos, sin = ops.rope_tables(4096, D, 1e4, dev)
+    pos = torch.randint(0, 4096, (tokens,), device=dev, generator=g, dtype=torch.int32)
+    slots = torch.randperm(nb * bs, generator=torch.Generator().manual_seed(2))[:tokens].int().to(dev)
+    slots[tokens // 2] = -1
+    a, b, (k1, v1), (k2, v2) = qkv.clone(), qkv.clone(), [p.clone() for p in pools], [p.clone() for p in pools]
+    lib, code, s = _native.lib(), _native.dtype_code(dtype), _native.stream_ptr(qkv.device)
+    _native.check(lib.tsb_rope_append_paged(a.data_ptr(), cos.data_ptr(), sin.data_ptr(), pos.data_ptr(), slots.data_ptr(), k1.data_ptr(), v1.data_ptr(),
+                                            tokens, H, Hkv, D, bs, code, s), "one")
+    b = ops.rope_qkv(b, cos, sin, num_heads=H, num_kv_heads=Hkv, head_dim=D, seq_len=1, positions=pos)
+    _native.check(lib.tsb_kv_append_paged(b.data_ptr(), cos.data_ptr(), sin.data_ptr(), pos.data_ptr(), slots.data_ptr(), k2.data_ptr(), v2.data_ptr(),
+                                          None, None, None, tokens, H, Hkv, D, bs, code, 0, s), "two")
+    for x, y in ((a, b), (k1, k2)):
+        assert bool(((x.float() - y.float()).abs() <= y.float().abs() * torch.finfo(dtype).eps + 1e-5).all())
+    assert torch.equal(a.view(tokens, -1, D)[:, H + Hkv:], b.view(tokens, -1, D)[:, H + Hkv:]) and torch.equal(v1, v2)
+    kept = torch.zeros(nb * bs, dtype=torch.bool, device=dev)
+    kept[slots[slots >= 0].long()] = True
+    rest = ~kept.view(nb, 1, bs, 1).expand_as(k1)
+    assert torch.equal(k1[rest], pools[0][rest])
+    assert lib.tsb_rope_append_paged(a.data_ptr() + 2, cos.data_ptr(), sin.data_ptr(), pos.data_ptr(), slots.data_ptr(), k1.data_ptr(), v1.data_ptr(),
+                                     tokens, H, Hkv, D, bs, code, s) == -2
+
+
 @pytest.mark.parametrize("size", [32, 4096, 148 * 32 * 256 * 32 + 32, 1 << 30])
 def test_zeroes(dev, size):
     from tesseract_b200 import _native
