@@ -25,10 +25,10 @@
 // Order of the MMAs of step i: dP_i, dV_i, S_{i+1}, dK_i, dQ_i. dP_i needs no probabilities and S_{i+1} no gradients, so that
 // P of step i + 1 is formed while dK_i, dQ_i and dP_{i+1} run, and dS_i while dV_i and S_{i+1} do.
 //
-// Measured, all of the backward pass (32 / 8 heads of 128, causal): 2 x 4096 tokens 1.89 -> 0.85 ms, 16384 tokens 13.6 -> 6.2 ms
-// (890 TFLOP/s) against four warps that went through scores, P, dS and dQ of a tile one after another; 16 heads of 64,
-// 4 x 1500 tokens, full: 382 -> 210 us. What bounds it now: the atomics of dQ for heads of 128 (above), for heads of 64 the chain from
-// scores over P and dS to the products (about 4200 clocks a step, of which the tensor core works 1280).
+// Measured, all of the backward pass (32 / 8 heads of 128, causal), L2 flushed: 2 x 4096 tokens 0.83 ms, 16384 tokens 6.2 ms (885 TFLOP/s; 0.87
+// and 6.4 with one lane's issue loops), against 1.89 and 13.6 for four warps that went through scores, P, dS and dQ of a tile one after another;
+// 16 heads of 64, 4 x 1500 tokens, full: 382 -> 208 us. What bounds it now: the atomics of dQ for heads of 128 (4.6 ms without them; the stores of dS
+// queue up behind them), for heads of 64 the two phases of the compute warps, P 1340 and dS 920 of 3200 clocks a step, of which the tensor core works 1280.
 //
 // A kernel before it writes delta_i = rowsum(dO_i * O_i) and lse_i in units of log 2 (+inf where a row sees no key or does not
 // exist: P is 0 there) and zeroes the scratch; one after it turns dQ into bf16.

@@ -695,7 +695,8 @@ flash_bounded_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 // shared memory and O in registers, which this kernel replaced (32 / 8 heads of 128, causal): 2 x 4096 tokens 580 -> 286 us (960
 // TFLOP/s), 16384 tokens 4.13 -> 1.99 ms (1110 TFLOP/s), 2 x 512 queries over 4608 keys 151 -> 81 us; 16 heads of 64, 4 x 1500 tokens,
 // full: 162 -> 79 us. (With a reference up to 2^8 behind: 268 us, 1.89 ms, 77, 76 us.) Every fourth exponential as a polynomial on the
-// FMA units was slower (16384 tokens: 1.80 -> 1.92 ms).
+// FMA units was slower (16384 tokens: 1.80 -> 1.92 ms). With issue loops that the whole warp walks, L2 flushed: 283 -> 273 us, 1.85 -> 1.81 ms,
+// 88 -> 86, 79.
 constexpr int kPairThreads = 384;
 // Registers per thread: 168 at the launch, 208 for the softmax warps and 88 for the rest after it (256 x 208 + 128 x 88 = 384 x 168).
 constexpr int kPairSoftmaxRegs = 208, kPairOtherRegs = 88;

@@ -505,7 +505,8 @@ __device__ __forceinline__ void umma_commit_pair_if(uint32_t pred, uint64_t* bar
 }
 
 template <bool A_MN, bool B_MN, typename OutT, bool ACCUM>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
+// (At most 168 registers where rows are added to, as for two CTAs on an SM: 33 K of them and a gradient all-reduce's 26 K go side by side.)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, ACCUM ? 2 : 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
                  OutT* __restrict__ C, int M, int N, int K, long long ldc, PairPlan pl, int by_tma, int* status) {
   using Cfg = PairTile;
@@ -673,15 +674,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       for (int half = 0; half < it.halves; ++half) {
         const int col0 = it.c0 + half * pl.n, cols = min(pl.n, N - col0);
         OutT* crow = C + static_cast<long long>(row) * ldc;
-        uint4 old[ACCUM && sizeof(OutT) == 2 ? 32 : 1];
-        if constexpr (ACCUM && sizeof(OutT) == 2) {
-          // what is added to comes while the products are formed (N is a multiple of 8 here)
-          if (by_tma && row < M) {
+        // What is added to comes while the products are formed, two pieces of 64 columns ahead (N is a multiple of 8 here). All four would
+        // take 64 registers more and the room of a gradient all-reduce's CTA beside this one.
+        uint4 old[2][ACCUM && sizeof(OutT) == 2 ? 8 : 1];
+        auto fetch = [&](int c) {
+          if constexpr (ACCUM && sizeof(OutT) == 2) {
+            if (by_tma && row < M) {
 #pragma unroll
-            for (int v = 0; v < 32; ++v)
-              if (v * 8 < cols) old[v] = *reinterpret_cast<const uint4*>(crow + col0 + v * 8);
+              for (int v = 0; v < 8; ++v)
+                if (c * 64 + v * 8 < cols) old[c & 1][v] = *reinterpret_cast<const uint4*>(crow + col0 + c * 64 + v * 8);
+            }
           }
-        }
+        };
+        fetch(0);
+        fetch(1);
         ok = mbar_wait_warp(&tmem_full_bar[acc], uses & 1, &cta_abort, status);
         if (!ok) break;
         tc_fence_after();
@@ -705,7 +711,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 #pragma unroll
                   for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(r[v * 8 + j]);
                   if constexpr (ACCUM) {
-                    const __nv_bfloat162* o2 = reinterpret_cast<const __nv_bfloat162*>(&old[c * 8 + v]);
+                    const __nv_bfloat162* o2 = reinterpret_cast<const __nv_bfloat162*>(&old[c & 1][v]);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                       const float2 of = __bfloat1622float2(o2[j]);
@@ -719,6 +725,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 }
                 *reinterpret_cast<uint4*>(piece + lane * 128 + ((v ^ (lane & 7)) << 4)) = o;
               }
+              if (c < 2) fetch(c + 2);
               fence_proxy_async_smem();
               __syncwarp();
               if (lane == 0) {
