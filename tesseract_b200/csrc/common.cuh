@@ -415,6 +415,20 @@ __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { retu
 template <>
 __device__ __forceinline__ __half from_f32<__half>(float v) { return __float2half_rn(v); }
 
+// Four adjacent pairs (x, y) of a row of T, rotated: (x c - y s, x s + y c). Which product of a sum is rounded by itself is written out: left to the
+// compiler, two kernels of the same lines rounded apart, and the last bits of a prompt's keys then depended on which of them had run. (16-bit rows:
+// the first pair apart from the other three, as the kernels have always had it.)
+template <typename T>
+__device__ __forceinline__ void rotate_pairs(float (&v)[8], float4 cos4, float4 sin4) {
+  const float c[4] = {cos4.x, cos4.y, cos4.z, cos4.w}, s[4] = {sin4.x, sin4.y, sin4.z, sin4.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float x = v[2 * i], y = v[2 * i + 1];
+    v[2 * i] = __fmaf_rn(x, c[i], -__fmul_rn(y, s[i]));
+    v[2 * i + 1] = sizeof(T) == 4 || i == 0 ? __fmaf_rn(y, c[i], __fmul_rn(x, s[i])) : __fmaf_rn(x, s[i], __fmul_rn(y, c[i]));
+  }
+}
+
 // Two fp32 operations in one instruction.
 __device__ __forceinline__ float2 mul_f32x2(float2 a, float2 b) {
   float2 d;

@@ -420,8 +420,8 @@ kv_append_kernel(T* __restrict__ qkv, const float* __restrict__ cos_t, const flo
 #pragma unroll
     for (int i = 0; i < EPL; i += 2) {
       const float a = x[i], b = x[i + 1], cc = c[i / 2], ss = s[i / 2];
-      x[i] = a * cc - b * ss;
-      x[i + 1] = a * ss + b * cc;
+      x[i] = __fmaf_rn(a, cc, -__fmul_rn(b, ss));          // (as in rotate_pairs; its lanes have one or two pairs each, all alike)
+      x[i + 1] = __fmaf_rn(b, cc, __fmul_rn(a, ss));
     }
   }
   if (is_q) {
@@ -684,13 +684,12 @@ rope_append_kernel(T* __restrict__ qkv, const float* __restrict__ cos_t, const f
       if (t >= tokens) continue;
       if (rotated) {
         T* e = reinterpret_cast<T*>(&raw[k]);
-        const float cc[4] = {c[k].x, c[k].y, c[k].z, c[k].w}, ss[4] = {s[k].x, s[k].y, s[k].z, s[k].w};
+        float x[8];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float x = to_f32<T>(e[2 * i]), y = to_f32<T>(e[2 * i + 1]);
-          e[2 * i] = from_f32<T>(x * cc[i] - y * ss[i]);
-          e[2 * i + 1] = from_f32<T>(x * ss[i] + y * cc[i]);
-        }
+        for (int i = 0; i < 8; ++i) x[i] = to_f32<T>(e[i]);
+        rotate_pairs<T>(x, c[k], s[k]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) e[i] = from_f32<T>(x[i]);
         *reinterpret_cast<uint4*>(qkv + (static_cast<long long>(t) * HT * kPieces + at) * 8) = raw[k];
       }
       if (kept && slot[k] >= 0) {

@@ -527,16 +527,13 @@ rope_qkv_kernel(T* __restrict__ qkv, const float* __restrict__ cos_t, const floa
     const long long t = th / heads_rot;
     const int p = pos ? pos[t] : pos_offset + static_cast<int>(t % seq_len);
     T* ptr = qkv + (t * heads_total + h) * D + v * 8;
-    float x[8], o[8];
+    float x[8];
     load8<T>(ptr, x);
     const float4 c = *reinterpret_cast<const float4*>(cos_t + static_cast<size_t>(p) * (D / 2) + v * 4);
     float4 s = *reinterpret_cast<const float4*>(sin_t + static_cast<size_t>(p) * (D / 2) + v * 4);
     s.x *= sign; s.y *= sign; s.z *= sign; s.w *= sign;
-    o[0] = x[0] * c.x - x[1] * s.x; o[1] = x[0] * s.x + x[1] * c.x;
-    o[2] = x[2] * c.y - x[3] * s.y; o[3] = x[2] * s.y + x[3] * c.y;
-    o[4] = x[4] * c.z - x[5] * s.z; o[5] = x[4] * s.z + x[5] * c.z;
-    o[6] = x[6] * c.w - x[7] * s.w; o[7] = x[6] * s.w + x[7] * c.w;
-    store8<T>(ptr, o);
+    rotate_pairs<T>(x, c, s);
+    store8<T>(ptr, x);
   }
 }
 
