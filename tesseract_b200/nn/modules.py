@@ -443,8 +443,9 @@ class TransformerBlock(Module):
                for t in (cos, sin)):
             return None
         order = (m1, qkv[0], o, m2, gu[0], down)
+        behind = (qkv[1], qkv[2], gu[1])
         return (x, residual, [weights[m] for m in order], [grads[m] for m in order], cos, sin, (B, S, W, H, Hkv, D, F),
-                (m1.eps, m2.eps, 1.0 / math.sqrt(D)), attn.causal)
+                (m1.eps, m2.eps, 1.0 / math.sqrt(D)), attn.causal, [t[m] for t in (weights, grads) for m in behind])
 
     def forward_fused(self, x: torch.Tensor, residual: Optional[torch.Tensor]):
         whole = self._whole(x, residual)

@@ -35,12 +35,34 @@ def _rows(t: torch.Tensor) -> torch.Tensor:
     return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
+_KEPT_TYPES = (torch.bfloat16, torch.uint8, torch.float32, torch.float32) + (torch.bfloat16,) * 10
+
+
+def _kept(t: torch.Tensor, size: int, dtype: torch.dtype, device: torch.device) -> torch.Tensor:
+    """A saved tensor that a hook has brought back somewhere else, as the kernels read it."""
+    if t.nbytes != size or t.dtype is not dtype or t.device != device:
+        raise RuntimeError(f"decoder_block: a saved tensor came back as {tuple(t.shape)} {t.dtype} on {t.device} instead of {size} bytes of {dtype} "
+                           f"on {device}")
+    return _rows(t)
+
+
+def _stack(*parts: torch.Tensor) -> torch.Tensor:
+    """Matrices one behind the other in memory: the first where they lie so, else a copy."""
+    at = parts[0].data_ptr()
+    for t in parts:
+        if t.data_ptr() != at:
+            return torch.cat(parts)
+        at += t.nbytes
+    return parts[0]
+
+
 class _BlockFn(torch.autograd.Function):
     """(out, res2) of x and the residual stream. ``weights`` and ``grads``: norm_1, q / k / v, o, norm_2, gate / up, down; of the stacked
-    ones the first, which the others follow in memory."""
+    ones the first, which the others (``behind``: k, v, up, and their gradients) follow in memory. All are saved: a hook that copies what is
+    saved copies the tensor it is given and not what lies behind it."""
 
     @staticmethod
-    def forward(ctx, x, res, norm_1, qkv, o, norm_2, gate_up, down, grads, cos, sin, shape, floats, causal):
+    def forward(ctx, x, res, norm_1, q, o, norm_2, gate, down, grads, behind, cos, sin, shape, floats, causal):
         ctx.set_materialize_grads(False)
         x = _rows(x)
         if res is not None:
@@ -48,29 +70,36 @@ class _BlockFn(torch.autograd.Function):
         shape, floats = _Shape(*shape), _Floats(*floats)
         saved = torch.empty(lib().tsb_block_saved_bytes(shape, int(res is not None)), device=x.device, dtype=torch.uint8)
         res2, out = torch.empty_like(x), torch.empty_like(x)
-        weights = (norm_1, qkv, o, norm_2, gate_up, down)
+        weights = (norm_1, q, o, norm_2, gate, down)
         args = _Fwd(x.data_ptr(), _ptr(res), *(w.data_ptr() for w in weights), cos.data_ptr(), sin.data_ptr(), saved.data_ptr(),
                     res2.data_ptr(), out.data_ptr())
         check(lib().tsb_block_forward(shape, args, floats, int(causal), stream_ptr(x.device)), "tsb_block_forward")
         _native.add_launches(LAUNCHES_FORWARD - 1)
-        ctx.save_for_backward(x if res is None else None, res2, saved, cos, sin, *weights)
-        ctx.grads, ctx.has_res, ctx.args = grads, res is not None, (shape, floats, causal)
+        keep = (res2, saved, cos, sin, *weights, *behind[:3]) + ((x,) if res is None else ())
+        ctx.save_for_backward(*keep)
+        ctx.kept = [t.data_ptr() for t in keep], [t.nbytes for t in keep]
+        ctx.grads, ctx.behind, ctx.has_res, ctx.args = grads, behind[3:], res is not None, (shape, floats, causal)
         return out, res2
 
     @staticmethod
     def backward(ctx, dout, dres2):
-        x, res2, saved, cos, sin, *weights = ctx.saved_tensors
+        back, (at, sizes) = ctx.saved_tensors, ctx.kept
+        if [t.data_ptr() for t in back] != at or [t.nbytes for t in back] != sizes or not all([t.is_contiguous() for t in back]):
+            device = (dres2 if dout is None else dout).device
+            back = [_kept(t, size, dtype, device) for t, size, dtype in zip(back, sizes, _KEPT_TYPES)]
+        res2, saved, cos, sin, norm_1, q, o, norm_2, gate, down, k, v, up, *x = back
+        weights = (norm_1, _stack(q, k, v), o, norm_2, _stack(gate, up), down)
         shape, floats, causal = ctx.args
         dout = torch.zeros_like(res2) if dout is None else _rows(dout)
         if dres2 is not None:
             dres2 = _rows(dres2)
         work = torch.empty(lib().tsb_block_work_bytes(shape), device=res2.device, dtype=torch.uint8)
         dx = torch.empty_like(res2)
-        args = _Bwd(_ptr(x), *(w.data_ptr() for w in weights), cos.data_ptr(), sin.data_ptr(), saved.data_ptr(), res2.data_ptr(),
+        args = _Bwd(x[0].data_ptr() if x else 0, *(w.data_ptr() for w in weights), cos.data_ptr(), sin.data_ptr(), saved.data_ptr(), res2.data_ptr(),
                     *(g.data_ptr() for g in ctx.grads), dout.data_ptr(), _ptr(dres2), work.data_ptr(), dx.data_ptr())
         check(lib().tsb_block_backward(shape, args, floats, int(ctx.has_res), int(causal), stream_ptr(res2.device)), "tsb_block_backward")
         _native.add_launches(LAUNCHES_BACKWARD - 1)
-        return (dx, dx if ctx.has_res else None) + (None,) * 12
+        return (dx, dx if ctx.has_res else None) + (None,) * 13
 
 
 def block_kernels_ok(x: torch.Tensor) -> bool:
@@ -78,7 +107,12 @@ def block_kernels_ok(x: torch.Tensor) -> bool:
     return _use_native(x) and _native_flash_available() and hasattr(lib(), "tsb_block_forward")
 
 
-def decoder_block(x, res, weights, grads, cos, sin, shape, floats, causal):
+def decoder_block(x, res, weights, grads, cos, sin, shape, floats, causal, behind=None):
     """``(out, x [+ res] + attention)``; ``shape`` is (B, S, W, H, Hkv, D, F), ``floats`` both norms' eps and the softmax scale. The gradients of
-    ``weights`` are added to ``grads``."""
-    return _BlockFn.apply(x, res, *weights, grads, cos, sin, shape, floats, causal)
+    ``weights`` are added to ``grads``; both, and ``behind``, as in ``_BlockFn``."""
+    if behind is None:
+        _, _, W, H, Hkv, D, F = shape
+        with torch.no_grad():
+            behind = [torch.as_strided(t[i], (rows, W), (W, 1), t[i].storage_offset() + first * W)
+                      for t in (weights, grads) for i, first, rows in ((1, H * D, Hkv * D), (1, (H + Hkv) * D, Hkv * D), (4, F, F))]
+    return _BlockFn.apply(x, res, *weights, grads, behind, cos, sin, shape, floats, causal)

@@ -1,4 +1,5 @@
 """Numerics of the native sm_100a kernels against plain PyTorch fp32 references of the same op."""
+import contextlib
 import math
 
 import pytest
@@ -555,6 +556,57 @@ def test_block_in_one_call_gives_what_its_modules_give(dev, width, heads, kv, ff
     assert results[0][0] == results[1][0]
     for a, b in zip(results[0][1], results[1][1]):
         assert float((a - b).norm()) <= 0.02 * float(b.norm()) + 1e-6
+
+
+def _run_block(blk, arena, x, res, dout, dres, around=contextlib.nullcontext()):
+    """(out, residual stream, gradients of x, of res and of the weights by name), everything cloned."""
+    arena.zero_grad()
+    x, res = (None if t is None else t.detach().clone().requires_grad_() for t in (x, res))
+    with around:
+        out, stream = blk.forward_fused(x, res)
+    ins = [x] if res is None else [x, res]
+    dx = torch.autograd.grad([out, stream], ins, [dout, dres])
+    return ([out.detach().clone(), stream.detach().clone()], list(dx),
+            {n: p.main_grad.clone() for n, p in blk.named_parameters()})
+
+
+def _block_inputs(dev, B, S, width, seed=0):
+    g = torch.Generator(device=dev).manual_seed(seed + S)
+    return [torch.randn(B, S, width, device=dev, generator=g).bfloat16() for _ in range(4)]
+
+
+BEHIND_DQ = ("norm_1.weight", "attn.q_proj.weight")      # gradients that depend on dQ
+
+
+def _same_blocks(a, b, exact):
+    """Of up to 256 keys the parts of dQ are two per value, whose sum is the same in either order; of more, only what does not depend on dQ is."""
+    assert all(torch.equal(s, t) for s, t in zip(a[0], b[0]))
+    for n in a[2]:
+        if exact or n not in BEHIND_DQ:
+            assert torch.equal(a[2][n], b[2][n]), n
+        else:
+            assert _rel_err(a[2][n], b[2][n].float()) < 2e-3, n
+    for s, t in zip(a[1], b[1]):
+        assert torch.equal(s, t) if exact else _rel_err(s, t.float()) < 2e-3
+
+
+@pytest.mark.parametrize("kind", ["copy", "host", "pinned", "off"])
+@pytest.mark.parametrize("has_res", [True, False])
+def test_block_under_hooks_on_saved_tensors(dev, kind, has_res):
+    """What is saved may come back somewhere else (activations kept on the host): weights with all their rows, from any address on."""
+    model, arena = _block_model(dev, 256, 2, 1, 688)
+    blk = model.layers[1]
+    x, res, dout, dres = _block_inputs(dev, 2, 150, 256)
+    res = res if has_res else None
+    assert blk._whole(x.requires_grad_(), res) is not None
+    want = _run_block(blk, arena, x, res, dout, dres)
+    moved = lambda t: torch.empty(t.numel() + 1, device=t.device, dtype=t.dtype)[1:].view(t.shape).copy_(t)
+    around = {"copy": lambda: torch.autograd.graph.saved_tensors_hooks(lambda t: t.detach().clone(), lambda t: t),
+              "off": lambda: torch.autograd.graph.saved_tensors_hooks(lambda t: t.detach(), moved),
+              "host": lambda: torch.autograd.graph.save_on_cpu(), "pinned": lambda: torch.autograd.graph.save_on_cpu(pin_memory=True)}[kind]()
+    got = _run_block(blk, arena, x, res, dout, dres, around)
+    _status_ok()
+    _same_blocks(got, want, exact=True)
 
 
 def test_block_runs_its_modules_where_they_are_not_plain(dev):
