@@ -14,6 +14,7 @@ from typing import Iterable
 import torch
 from torch import nn
 
+from .. import _native
 from .._native import check, lib, stream_ptr
 
 _ALIGN_ELEMS = 128  # every parameter starts on a 256-byte (bf16) / 512-byte (fp32) boundary
@@ -67,7 +68,9 @@ class ParamArena:
     def _zero(self) -> None:
         g = self.grad
         size = g.numel() * g.element_size()
-        if g.is_cuda and size % 32 == 0 and g.data_ptr() % 32 == 0 and hasattr(lib(), "tsb_zero"):
+        # (kernels go to the current device: a buffer on another one, or a checkout without a built library, is torch's to clear)
+        if (g.is_cuda and size % 32 == 0 and g.data_ptr() % 32 == 0 and g.device.index == torch.cuda.current_device() and _native.available()
+                and hasattr(lib(), "tsb_zero")):
             check(lib().tsb_zero(g.data_ptr(), size, stream_ptr(g.device)), "tsb_zero")
         else:
             g.zero_()

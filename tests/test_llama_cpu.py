@@ -1,6 +1,7 @@
 """Tiny Llama on CPU (fp32): arena + fused loss parity with plain autograd, one Adam step, config parsing."""
 import json
 
+import pytest
 import torch
 
 from tesseract_b200.models import LlamaConfig, LlamaModel, llama_local_to_hf_name
@@ -82,3 +83,47 @@ def test_config_from_json():
     assert cfg.vocab_size == 100 and cfg.num_experts == 4 and cfg.dtype == torch.bfloat16
     assert cfg.rope_theta == 5e5 and cfg.tie_word_embeddings and cfg.eos_token_id == 7
     assert cfg.kv_heads() == cfg.num_attention_heads
+
+
+@pytest.mark.parametrize("device,built,shift,native", [(0, True, 0, True), (1, True, 0, False), (0, False, 0, False), (0, True, 16, False)])
+def test_gradients_are_cleared_on_their_own_device(monkeypatch, device, built, shift, native):
+    """The kernel runs on the current device (0 here): a gradient buffer elsewhere, off 32 bytes or without a library is cleared by torch."""
+    from tesseract_b200.optim import arena as module
+
+    class Grad:
+        is_cuda, cleared = True, False
+
+        def numel(self):
+            return 128
+
+        def element_size(self):
+            return 2
+
+        def data_ptr(self):
+            return 1 << 20 | shift
+
+        def zero_(self):
+            self.cleared = True
+
+    calls = []
+
+    class Library:
+        def tsb_zero(self, at, size, stream):
+            calls.append((at, size))
+            return 0
+
+    def lib():
+        if not built:
+            raise RuntimeError("not built")
+        return Library()
+
+    grad = Grad()
+    grad.device = torch.device("cuda", device)
+    a = ParamArena.__new__(ParamArena)
+    a.grad, a.params = grad, []
+    monkeypatch.setattr(module, "lib", lib)
+    monkeypatch.setattr(module, "stream_ptr", lambda d: 0)
+    monkeypatch.setattr("tesseract_b200._native.available", lambda: built)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    a.zero_grad()
+    assert grad.cleared is not native and calls == ([(1 << 20, 256)] if native else [])
