@@ -6,13 +6,16 @@
 // kernels). From here: 1.53 ms.
 #include "common.cuh"
 
+#include <algorithm>
+
 TSB_EXPORT int tsb_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* h_out, float* rstd, int rows, int D, float eps,
                                int dtype, void* stream);
 TSB_EXPORT int tsb_rmsnorm_bwd_parts(int rows);
 TSB_EXPORT int tsb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx, void* dw,
                                float* partial, int rows, int D, int accumulate_dw, int dtype, void* stream);
 TSB_EXPORT int tsb_swiglu_fwd(const void* gate_up, void* out, long long rows, int F, int dtype, void* stream);
-TSB_EXPORT int tsb_swiglu_bwd(const void* dout, const void* gate_up, void* dgate_up, long long rows, int F, int dtype, void* stream);
+TSB_EXPORT int tsb_swiglu_bwd_rows(const void* dout, long long ld_dout, const void* gate_up, void* dgate_up, long long rows, int F, int dtype,
+                                   void* stream);
 TSB_EXPORT int tsb_rope_qkv(void* qkv, const float* cos_t, const float* sin_t, const int* pos, long long tokens, int seq_len, int pos_offset,
                             int heads_rot, int heads_total, int D, float sign, int dtype, void* stream);
 TSB_EXPORT int tsb_flash_fwd(const void* q, const void* k, const void* v, void* o, float* lse, int B, int Sq, int Sk, int H, int Hkv, int D,
@@ -53,46 +56,48 @@ struct Cut {
   }
 };
 
-// What the forward pass leaves for the backward pass.
+// What the forward pass leaves for the backward pass, in two pieces: the second is done with halfway and given back then.
 struct Saved {
   uint8_t *h1, *res1, *qkv, *o, *h2, *gu, *act;
   float *rstd1, *rstd2, *lse;
-  long long bytes;
-  Saved(const BlockShape& s, void* base, bool has_res) {
-    Cut c{static_cast<uint8_t*>(base)};
+  long long bytes, mid_bytes;
+  Saved(const BlockShape& s, void* base, void* mid, bool has_res) {
+    Cut c{static_cast<uint8_t*>(base)}, m{static_cast<uint8_t*>(mid)};
     const long long T = s.rows();
     h1 = c.take(T * s.W * 2);
     res1 = has_res ? c.take(T * s.W * 2) : nullptr;
     qkv = c.take(T * s.packed() * 2);
     o = c.take(T * s.W * 2);
     h2 = c.take(T * s.W * 2);
-    gu = c.take(T * 2 * s.F * 2);
-    act = c.take(T * s.F * 2);
+    gu = m.take(T * 2 * s.F * 2);
+    act = m.take(T * s.F * 2);
     rstd1 = reinterpret_cast<float*>(c.take(T * 4));
     rstd2 = reinterpret_cast<float*>(c.take(T * 4));
     lse = reinterpret_cast<float*>(c.take(T * s.H * 4));
     bytes = c.at;
+    mid_bytes = m.at;
   }
 };
 
-// What the backward pass needs meanwhile: what the attention half needs lies where the gradients of the feed-forward half were.
+// What the backward pass needs meanwhile, in two pieces. No more is held at any time than the modules hold one by one (16384 tokens, width 4096,
+// 14336 between: 6.9 GB a step over the weights, where one piece for all and a buffer for each gradient took 7.6):
+//   wide   the gradient of gate and up, in which that of the activation is formed first (in the columns of gate, which SwiGLU's backward pass
+//          reads and writes in place); then what attention adds dQ up in; then the gradient of norm_1's output.
+//   rest   the gradient of the stream between the halves, of q / k / v, and the norms' sums. Taken when `mid` has been given back.
+// The gradients of norm_2's output and of attention's lie in dx, which is filled last.
 struct Work {
-  uint8_t *da, *dact, *dgu, *d_o, *dqkv, *dh1, *scratch;
+  uint8_t *wide, *da, *dqkv;
   float* partial;
-  long long bytes;
-  Work(const BlockShape& s, void* base) {
-    Cut c{static_cast<uint8_t*>(base)};
+  long long wide_bytes, rest_bytes;
+  Work(const BlockShape& s, void* wide_base, void* rest_base) {
+    Cut c{static_cast<uint8_t*>(rest_base)};
     const long long T = s.rows();
+    wide = static_cast<uint8_t*>(wide_base);
+    wide_bytes = std::max({T * 2 * s.F * 2, T * s.W * 2, tsb_flash_bwd_scratch_bytes(s.B, s.S, s.H, s.D)});
     da = c.take(T * s.W * 2);
-    partial = reinterpret_cast<float*>(c.take(static_cast<long long>(tsb_rmsnorm_bwd_parts(static_cast<int>(T))) * s.W * 4));
-    Cut f = c;
-    dact = f.take(T * s.F * 2);
-    dgu = f.take(T * 2 * s.F * 2);
-    d_o = c.take(T * s.W * 2);
     dqkv = c.take(T * s.packed() * 2);
-    dh1 = c.take(T * s.W * 2);
-    scratch = c.take(tsb_flash_bwd_scratch_bytes(s.B, s.S, s.H, s.D));
-    bytes = f.at > c.at ? f.at : c.at;
+    partial = reinterpret_cast<float*>(c.take(static_cast<long long>(tsb_rmsnorm_bwd_parts(static_cast<int>(T))) * s.W * 4));
+    rest_bytes = c.at;
   }
 };
 
@@ -107,27 +112,31 @@ T* ptr(long long v) { return reinterpret_cast<T*>(v); }
 }  // namespace tsb
 
 // Host arrays. shape: B, S, W, H, Hkv, D, F (W = H * D; D 64 or 128; F a multiple of 8).
-// Bytes that a forward call keeps in `saved`, and that a backward call needs in `work`; -2 for other shapes.
-TSB_EXPORT long long tsb_block_saved_bytes(const long long* shape, int has_res) {
-  const tsb::BlockShape s = tsb::shape_of(shape);
-  return s.ok() ? tsb::Saved(s, nullptr, has_res != 0).bytes : -2;
-}
-TSB_EXPORT long long tsb_block_work_bytes(const long long* shape) {
-  const tsb::BlockShape s = tsb::shape_of(shape);
-  return s.ok() ? tsb::Work(s, nullptr).bytes : -2;
+// bytes: what a forward call keeps in `saved` and in `mid`, what a backward call needs in `wide` and in `rest`. -2 for other shapes.
+TSB_EXPORT int tsb_block_bytes(const long long* shape, int has_res, long long* bytes) {
+  using namespace tsb;
+  const BlockShape s = shape_of(shape);
+  if (!s.ok()) return -2;
+  const Saved k(s, nullptr, nullptr, has_res != 0);
+  const Work w(s, nullptr, nullptr);
+  bytes[0] = k.bytes;
+  bytes[1] = k.mid_bytes;
+  bytes[2] = w.wide_bytes;
+  bytes[3] = w.rest_bytes;
+  return 0;
 }
 
 // out = down(silu(gate) * up) of the normed stream; res2 = x [+ res] + o_proj(attention). All bf16, contiguous, 16-byte aligned.
-// p: x, res (0: none), norm_1, qkv weight, o weight, norm_2, gate and up weight, down weight, cos, sin, saved, res2, out.
-// f: eps of norm_1, eps of norm_2, softmax scale. Rows of weights are stacked (q, k, v; gate, up). `saved`: see above, 256-byte aligned.
+// p: x, res (0: none), norm_1, qkv weight, o weight, norm_2, gate and up weight, down weight, cos, sin, saved, mid, res2, out.
+// f: eps of norm_1, eps of norm_2, softmax scale. Rows of weights are stacked (q, k, v; gate, up).
 TSB_EXPORT int tsb_block_forward(const long long* shape, const long long* p, const float* f, int causal, void* stream) {
   using namespace tsb;
   const BlockShape s = shape_of(shape);
   if (!s.ok()) return -2;
-  const Saved k(s, ptr(p[10]), p[1] != 0);
+  const Saved k(s, ptr(p[10]), ptr(p[11]), p[1] != 0);
   const int T = static_cast<int>(s.rows()), N = static_cast<int>(s.packed()), W = s.W, F = s.F, D = s.D;
   const long long row = N, seq = static_cast<long long>(s.S) * N, hd = static_cast<long long>(s.H) * D, vd = hd + static_cast<long long>(s.Hkv) * D;
-  void *res2 = ptr(p[11]), *out = ptr(p[12]);
+  void *res2 = ptr(p[12]), *out = ptr(p[13]);
   auto product = [&](const void* x, long long w, void* y, int cols, int depth) {
     return tsb_gemm_bf16(x, ptr(w), y, T, cols, depth, depth, depth, cols, 0, 0, 0, 0, 0, 0, stream);
   };
@@ -148,39 +157,58 @@ TSB_EXPORT int tsb_block_forward(const long long* shape, const long long* p, con
   return product(k.act, p[7], out, W, F);
 }
 
-// Gradients of the above. p: x (where there was no res; else unused), norm_1, qkv, o, norm_2, gate and up, down (weights), cos, sin, saved,
-// res2, gradients of norm_1, qkv, o, norm_2, gate and up, down (added to; bf16), dout, dres2 (0: none), work, dx (of x and of res).
+namespace tsb {
+namespace {
+
+int product_input(const void* dy, long long weight, void* d, int rows, int outs, int ins, long long ldd, void* stream) {      // d = dy W
+  return tsb_gemm_bf16(dy, ptr(weight), d, rows, ins, outs, outs, ins, ldd, 0, 1, 0, 0, 0, 0, stream);
+}
+int product_weight(const void* dy, const void* x, long long d, int rows, int outs, int ins, void* stream) {                   // dW += dy^T x
+  return tsb_gemm_bf16(dy, x, ptr(d), outs, ins, rows, outs, ins, ins, 1, 1, 0, 1, 0, 0, stream);
+}
+
+}  // namespace
+}  // namespace tsb
+
+// Gradients of the above, first part: from the block's output to gate and up. What `mid` holds is not needed after it.
+// p: down weight, mid, gradient of down (added to; bf16), dout, wide.
+TSB_EXPORT int tsb_block_backward_down(const long long* shape, const long long* p, void* stream) {
+  using namespace tsb;
+  const BlockShape s = shape_of(shape);
+  if (!s.ok()) return -2;
+  const Saved k(s, nullptr, ptr(p[1]), false);
+  const int T = static_cast<int>(s.rows()), W = s.W, F = s.F;
+  const void* dout = ptr(p[3]);
+  void* dgu = ptr(p[4]);
+  int rc = product_input(dout, p[0], dgu, T, W, F, 2LL * F, stream);
+  if (rc) return rc;
+  if ((rc = product_weight(dout, k.act, p[2], T, W, F, stream))) return rc;
+  return tsb_swiglu_bwd_rows(dgu, 2LL * F, k.gu, dgu, T, F, kBf16, stream);
+}
+
+// The rest. p: x (where there was no res; else unused), norm_1, qkv, o, norm_2, gate and up (weights), cos, sin, saved, res2, gradients of norm_1,
+// qkv, o, norm_2, gate and up (added to; bf16), dres2 (0: none), wide (as the first part left it), rest, dx (of x and of res). f: as forward.
 TSB_EXPORT int tsb_block_backward(const long long* shape, const long long* p, const float* f, int has_res, int causal, void* stream) {
   using namespace tsb;
   const BlockShape s = shape_of(shape);
   if (!s.ok()) return -2;
-  const Saved k(s, ptr(p[9]), has_res != 0);
-  const Work w(s, ptr(p[19]));
+  const Saved k(s, ptr(p[8]), nullptr, has_res != 0);
+  const Work w(s, ptr(p[16]), ptr(p[17]));
   const int T = static_cast<int>(s.rows()), N = static_cast<int>(s.packed()), W = s.W, F = s.F, D = s.D;
   const long long row = N, seq = static_cast<long long>(s.S) * N, hd = static_cast<long long>(s.H) * D, vd = hd + static_cast<long long>(s.Hkv) * D;
-  void* dx = ptr(p[20]);
-  auto input = [&](const void* dy, long long weight, void* d, int outs, int ins) {                // d = dy W
-    return tsb_gemm_bf16(dy, ptr(weight), d, T, ins, outs, outs, ins, ins, 0, 1, 0, 0, 0, 0, stream);
-  };
-  auto weight = [&](const void* dy, const void* x, long long d, int outs, int ins) {              // dW += dy^T x
-    return tsb_gemm_bf16(dy, x, ptr(d), outs, ins, T, outs, ins, ins, 1, 1, 0, 1, 0, 0, stream);
-  };
-  const void* dout = ptr(p[17]);
-  int rc = input(dout, p[6], w.dact, W, F);
+  void *dx = ptr(p[18]), *dh2 = dx, *d_o = dx, *dh1 = w.wide;
+  int rc = product_input(w.wide, p[5], dh2, T, 2 * F, W, W, stream);
   if (rc) return rc;
-  if ((rc = weight(dout, k.act, p[16], W, F))) return rc;
-  if ((rc = tsb_swiglu_bwd(w.dact, k.gu, w.dgu, T, F, kBf16, stream))) return rc;
-  if ((rc = input(w.dgu, p[5], dx, 2 * F, W))) return rc;                      // (dx, free until the end, has the gradient of norm_2's output)
-  if ((rc = weight(w.dgu, k.h2, p[15], 2 * F, W))) return rc;
-  if ((rc = tsb_rmsnorm_bwd(dx, ptr(p[10]), ptr(p[4]), k.rstd2, ptr(p[18]), w.da, ptr(p[14]), w.partial, T, W, 1, kBf16, stream))) return rc;
-  if ((rc = input(w.da, p[3], w.d_o, W, W))) return rc;
-  if ((rc = weight(w.da, k.o, p[13], W, W))) return rc;
-  rc = tsb_flash_bwd(w.d_o, k.qkv, k.qkv + hd * 2, k.qkv + vd * 2, k.o, k.lse, w.dqkv, w.dqkv + hd * 2, w.dqkv + vd * 2, w.scratch, s.B, s.S, s.S,
+  if ((rc = product_weight(w.wide, k.h2, p[14], T, 2 * F, W, stream))) return rc;
+  if ((rc = tsb_rmsnorm_bwd(dh2, ptr(p[9]), ptr(p[4]), k.rstd2, ptr(p[15]), w.da, ptr(p[13]), w.partial, T, W, 1, kBf16, stream))) return rc;
+  if ((rc = product_input(w.da, p[3], d_o, T, W, W, W, stream))) return rc;
+  if ((rc = product_weight(w.da, k.o, p[12], T, W, W, stream))) return rc;
+  rc = tsb_flash_bwd(d_o, k.qkv, k.qkv + hd * 2, k.qkv + vd * 2, k.o, k.lse, w.dqkv, w.dqkv + hd * 2, w.dqkv + vd * 2, w.wide, s.B, s.S, s.S,
                      s.H, s.Hkv, D, seq, row, D, seq, row, D, seq, row, D, seq, row, D, f[2], causal, stream);
   if (rc) return rc;
-  rc = tsb_rope_qkv(w.dqkv, ptr<float>(p[7]), ptr<float>(p[8]), nullptr, T, s.S, 0, s.H + s.Hkv, s.H + 2 * s.Hkv, D, -1.f, kBf16, stream);
+  rc = tsb_rope_qkv(w.dqkv, ptr<float>(p[6]), ptr<float>(p[7]), nullptr, T, s.S, 0, s.H + s.Hkv, s.H + 2 * s.Hkv, D, -1.f, kBf16, stream);
   if (rc) return rc;
-  if ((rc = input(w.dqkv, p[2], w.dh1, N, W))) return rc;
-  if ((rc = weight(w.dqkv, k.h1, p[12], N, W))) return rc;
-  return tsb_rmsnorm_bwd(w.dh1, has_res ? k.res1 : ptr(p[0]), ptr(p[1]), k.rstd1, w.da, dx, ptr(p[11]), w.partial, T, W, 1, kBf16, stream);
+  if ((rc = product_input(w.dqkv, p[2], dh1, T, N, W, W, stream))) return rc;
+  if ((rc = product_weight(w.dqkv, k.h1, p[11], T, N, W, stream))) return rc;
+  return tsb_rmsnorm_bwd(dh1, has_res ? k.res1 : ptr(p[0]), ptr(p[1]), k.rstd1, w.da, dx, ptr(p[10]), w.partial, T, W, 1, kBf16, stream);
 }

@@ -418,12 +418,12 @@ swiglu_fwd_wide_kernel(const T* __restrict__ gate_up, T* __restrict__ out, int r
 }
 template <typename T>
 __global__ void __launch_bounds__(kGluThreads)
-swiglu_bwd_wide_kernel(const T* __restrict__ dout, const T* __restrict__ gate_up, T* __restrict__ dgate_up, int rows, int F) {
+swiglu_bwd_wide_kernel(const T* dout, long long ld_dout, const T* __restrict__ gate_up, T* dgate_up, int rows, int F) {
   const int c = (blockIdx.x * kGluThreads + threadIdx.x) * 16;
   if (c >= F) return;
   for (int row = blockIdx.y; row < rows; row += gridDim.y) {
     const size_t at = static_cast<size_t>(row) * 2 * F + c;
-    const Bytes32 g = ld_global_32(gate_up + at), u = ld_global_32(gate_up + at + F), d = ld_global_32(dout + static_cast<size_t>(row) * F + c);
+    const Bytes32 g = ld_global_32(gate_up + at), u = ld_global_32(gate_up + at + F), d = ld_global_32(dout + row * ld_dout + c);
     float gf[16], uf[16], df[16];
     unpack16<T>(g, gf);
     unpack16<T>(u, uf);
@@ -448,11 +448,11 @@ inline dim3 glu_wide_grid(long long rows, int F, int rows_each) {
   return dim3(gx, static_cast<unsigned>(std::min<long long>({want, need, 65535})));
 }
 
-// d(gate_up) from d(out): dg = dout*u*s*(1+g*(1-s)), du = dout*g*s with s = sigmoid(g).
+// d(gate_up) from d(out): dg = dout*u*s*(1+g*(1-s)), du = dout*g*s with s = sigmoid(g). Rows of dout are ld_dout apart, and dout may lie in the
+// columns of gate of dgate_up (in all three kernels): a thread reads what it overwrites, and nothing else of it, before it does.
 template <typename T>
 __global__ void __launch_bounds__(256)
-swiglu_bwd_kernel(const T* __restrict__ dout, const T* __restrict__ gate_up, T* __restrict__ dgate_up, long long rows,
-                  int F) {
+swiglu_bwd_kernel(const T* dout, long long ld_dout, const T* __restrict__ gate_up, T* dgate_up, long long rows, int F) {
   const long long nvec = rows * (F / 8);
   const int vpr = F / 8;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < nvec;
@@ -462,7 +462,7 @@ swiglu_bwd_kernel(const T* __restrict__ dout, const T* __restrict__ gate_up, T* 
     float g[8], u[8], d[8], dg[8], du[8];
     load8<T>(gate_up + row * 2 * F + c, g);
     load8<T>(gate_up + row * 2 * F + F + c, u);
-    load8<T>(dout + row * F + c, d);
+    load8<T>(dout + row * ld_dout + c, d);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const float s = 1.f / (1.f + __expf(-g[j]));
@@ -476,11 +476,11 @@ swiglu_bwd_kernel(const T* __restrict__ dout, const T* __restrict__ gate_up, T* 
 
 template <typename T, int UNR>
 __global__ void __launch_bounds__(256)
-swiglu_bwd_rows_kernel(const T* __restrict__ dout, const T* __restrict__ gate_up, T* __restrict__ dgate_up, int rows, int F) {
+swiglu_bwd_rows_kernel(const T* dout, long long ld_dout, const T* __restrict__ gate_up, T* dgate_up, int rows, int F) {
   const int vpr = F / 8;
   for (int row = blockIdx.y; row < rows; row += gridDim.y) {
     const T* gp = gate_up + static_cast<size_t>(row) * 2 * F;
-    const T* dp = dout + static_cast<size_t>(row) * F;
+    const T* dp = dout + row * ld_dout;
     T* op = dgate_up + static_cast<size_t>(row) * 2 * F;
     for (int v0 = (blockIdx.x * blockDim.x + threadIdx.x) * UNR; v0 < vpr; v0 += gridDim.x * blockDim.x * UNR) {
       float g[UNR][8], u[UNR][8], d[UNR][8];
@@ -725,22 +725,23 @@ TSB_EXPORT int tsb_swiglu_fwd(const void* gate_up, void* out, long long rows, in
   return static_cast<int>(cudaGetLastError());
 }
 
-TSB_EXPORT int tsb_swiglu_bwd(const void* dout, const void* gate_up, void* dgate_up, long long rows, int F, int dtype,
-                              void* stream) {
-  if (rows <= 0 || F <= 0 || F % 8) return -2;
+// Rows of dout are ld_dout values apart (a multiple of 8); dout may be dgate_up itself, with rows 2F apart.
+TSB_EXPORT int tsb_swiglu_bwd_rows(const void* dout, long long ld_dout, const void* gate_up, void* dgate_up, long long rows, int F, int dtype,
+                                   void* stream) {
+  if (rows <= 0 || F <= 0 || F % 8 || ld_dout < F || ld_dout % 8) return -2;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   static const int mode = [] { const char* e = getenv("TESSERACT_SWIGLU"); return e ? atoi(e) : 2; }();
   if (mode == 0 || rows > 0x7fffffffLL) {
     const int grid = tsb::ew_grid(rows * (F / 8), 256);
     TSB_DISPATCH_FLOAT(dtype, (tsb::swiglu_bwd_kernel<T><<<grid, 256, 0, s>>>(
-                                  static_cast<const T*>(dout), static_cast<const T*>(gate_up),
+                                  static_cast<const T*>(dout), ld_dout, static_cast<const T*>(gate_up),
                                   static_cast<T*>(dgate_up), rows, F)));
     return static_cast<int>(cudaGetLastError());
   }
-  if (tsb::glu_wide_ok(dtype, F, gate_up, dgate_up, dout)) {
+  if (ld_dout % 16 == 0 && tsb::glu_wide_ok(dtype, F, gate_up, dgate_up, dout)) {
     const dim3 grid = tsb::glu_wide_grid(rows, F, 1);
-    if (dtype == 1) tsb::swiglu_bwd_wide_kernel<__nv_bfloat16><<<grid, tsb::kGluThreads, 0, s>>>(static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(gate_up), static_cast<__nv_bfloat16*>(dgate_up), static_cast<int>(rows), F);
-    else if (dtype == 2) tsb::swiglu_bwd_wide_kernel<__half><<<grid, tsb::kGluThreads, 0, s>>>(static_cast<const __half*>(dout), static_cast<const __half*>(gate_up), static_cast<__half*>(dgate_up), static_cast<int>(rows), F);
+    if (dtype == 1) tsb::swiglu_bwd_wide_kernel<__nv_bfloat16><<<grid, tsb::kGluThreads, 0, s>>>(static_cast<const __nv_bfloat16*>(dout), ld_dout, static_cast<const __nv_bfloat16*>(gate_up), static_cast<__nv_bfloat16*>(dgate_up), static_cast<int>(rows), F);
+    else if (dtype == 2) tsb::swiglu_bwd_wide_kernel<__half><<<grid, tsb::kGluThreads, 0, s>>>(static_cast<const __half*>(dout), ld_dout, static_cast<const __half*>(gate_up), static_cast<__half*>(dgate_up), static_cast<int>(rows), F);
     else return -2;
     return static_cast<int>(cudaGetLastError());
   }
@@ -751,9 +752,12 @@ TSB_EXPORT int tsb_swiglu_bwd(const void* dout, const void* gate_up, void* dgate
   if (gy > 65535) gy = 65535;
   const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy));
   TSB_DISPATCH_FLOAT(dtype, (tsb::swiglu_bwd_rows_kernel<T, 2><<<grid, 256, 0, s>>>(
-                                static_cast<const T*>(dout), static_cast<const T*>(gate_up),
+                                static_cast<const T*>(dout), ld_dout, static_cast<const T*>(gate_up),
                                 static_cast<T*>(dgate_up), static_cast<int>(rows), F)));
   return static_cast<int>(cudaGetLastError());
+}
+TSB_EXPORT int tsb_swiglu_bwd(const void* dout, const void* gate_up, void* dgate_up, long long rows, int F, int dtype, void* stream) {
+  return tsb_swiglu_bwd_rows(dout, F, gate_up, dgate_up, rows, F, dtype, stream);
 }
 
 // In-place adjacent-pair RoPE on the first `heads_rot` heads of every token of a packed [tokens,

@@ -13,15 +13,14 @@ from .attention import _native_flash_available
 from .gemm import _use_native
 
 _native.register_signatures({
-    "tsb_block_saved_bytes": [_native.P, _native.I],
-    "tsb_block_work_bytes": [_native.P],
+    "tsb_block_bytes": [_native.P, _native.I, _native.P],
     "tsb_block_forward": [_native.P, _native.P, _native.P, _native.I, _native.P],
+    "tsb_block_backward_down": [_native.P, _native.P, _native.P],
     "tsb_block_backward": [_native.P, _native.P, _native.P, _native.I, _native.I, _native.P],
 })
-_native._RESTYPES["tsb_block_saved_bytes"] = _native._RESTYPES["tsb_block_work_bytes"] = _native.L
 
-_Shape, _Floats = ctypes.c_longlong * 7, ctypes.c_float * 3
-_Fwd, _Bwd = ctypes.c_longlong * 13, ctypes.c_longlong * 21
+_Shape, _Floats, _Bytes = ctypes.c_longlong * 7, ctypes.c_float * 3, ctypes.c_longlong * 4
+_Fwd, _Down, _Bwd = ctypes.c_longlong * 14, ctypes.c_longlong * 5, ctypes.c_longlong * 19
 LAUNCHES_FORWARD, LAUNCHES_BACKWARD = 9, 18
 
 
@@ -35,7 +34,8 @@ def _rows(t: torch.Tensor) -> torch.Tensor:
     return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
-_KEPT_TYPES = (torch.bfloat16, torch.uint8, torch.float32, torch.float32) + (torch.bfloat16,) * 10
+_KEPT_TYPES = (torch.bfloat16, torch.uint8, torch.uint8, torch.float32, torch.float32) + (torch.bfloat16,) * 10
+_CAN_LET_GO = hasattr(torch.autograd.function.BackwardCFunction, "maybe_clear_saved_tensors")
 
 
 def _kept(t: torch.Tensor, size: int, dtype: torch.dtype, device: torch.device) -> torch.Tensor:
@@ -68,17 +68,21 @@ class _BlockFn(torch.autograd.Function):
         if res is not None:
             res = _rows(res)
         shape, floats = _Shape(*shape), _Floats(*floats)
-        saved = torch.empty(lib().tsb_block_saved_bytes(shape, int(res is not None)), device=x.device, dtype=torch.uint8)
+        sizes = _Bytes()
+        if lib().tsb_block_bytes(shape, int(res is not None), sizes) != 0:
+            raise ValueError("decoder_block: a shape that the kernels do not serve")
+        saved = torch.empty(sizes[0], device=x.device, dtype=torch.uint8)
+        mid = torch.empty(sizes[1], device=x.device, dtype=torch.uint8)
         res2, out = torch.empty_like(x), torch.empty_like(x)
         weights = (norm_1, q, o, norm_2, gate, down)
         args = _Fwd(x.data_ptr(), _ptr(res), *(w.data_ptr() for w in weights), cos.data_ptr(), sin.data_ptr(), saved.data_ptr(),
-                    res2.data_ptr(), out.data_ptr())
+                    mid.data_ptr(), res2.data_ptr(), out.data_ptr())
         check(lib().tsb_block_forward(shape, args, floats, int(causal), stream_ptr(x.device)), "tsb_block_forward")
         _native.add_launches(LAUNCHES_FORWARD - 1)
-        keep = (res2, saved, cos, sin, *weights, *behind[:3]) + ((x,) if res is None else ())
+        keep = (res2, saved, mid, cos, sin, *weights, *behind[:3]) + ((x,) if res is None else ())
         ctx.save_for_backward(*keep)
         ctx.kept = [t.data_ptr() for t in keep], [t.nbytes for t in keep]
-        ctx.grads, ctx.behind, ctx.has_res, ctx.args = grads, behind[3:], res is not None, (shape, floats, causal)
+        ctx.grads, ctx.behind, ctx.has_res, ctx.args = grads, behind[3:], res is not None, (shape, floats, causal, sizes)
         return out, res2
 
     @staticmethod
@@ -87,18 +91,27 @@ class _BlockFn(torch.autograd.Function):
         if [t.data_ptr() for t in back] != at or [t.nbytes for t in back] != sizes or not all([t.is_contiguous() for t in back]):
             device = (dres2 if dout is None else dout).device
             back = [_kept(t, size, dtype, device) for t, size, dtype in zip(back, sizes, _KEPT_TYPES)]
-        res2, saved, cos, sin, norm_1, q, o, norm_2, gate, down, k, v, up, *x = back
-        weights = (norm_1, _stack(q, k, v), o, norm_2, _stack(gate, up), down)
-        shape, floats, causal = ctx.args
+        res2, saved, mid, cos, sin, norm_1, q, o, norm_2, gate, down, k, v, up, *x = back
+        shape, floats, causal, (_, _, wide_bytes, rest_bytes) = ctx.args
+        grads = [g.data_ptr() for g in ctx.grads]
         dout = torch.zeros_like(res2) if dout is None else _rows(dout)
         if dres2 is not None:
             dres2 = _rows(dres2)
-        work = torch.empty(lib().tsb_block_work_bytes(shape), device=res2.device, dtype=torch.uint8)
+        stream = stream_ptr(res2.device)
+        wide = torch.empty(wide_bytes, device=res2.device, dtype=torch.uint8)
+        args = _Down(down.data_ptr(), mid.data_ptr(), grads.pop(), dout.data_ptr(), wide.data_ptr())
+        check(lib().tsb_block_backward_down(shape, args, stream), "tsb_block_backward_down")
+        # unless the graph is kept for another pass, the widest activations go back to the allocator here, as they do between modules
+        back = mid = None
+        if _CAN_LET_GO:
+            ctx.maybe_clear_saved_tensors()
+        rest = torch.empty(rest_bytes, device=res2.device, dtype=torch.uint8)
         dx = torch.empty_like(res2)
+        weights = (norm_1, _stack(q, k, v), o, norm_2, _stack(gate, up))
         args = _Bwd(x[0].data_ptr() if x else 0, *(w.data_ptr() for w in weights), cos.data_ptr(), sin.data_ptr(), saved.data_ptr(), res2.data_ptr(),
-                    *(g.data_ptr() for g in ctx.grads), dout.data_ptr(), _ptr(dres2), work.data_ptr(), dx.data_ptr())
-        check(lib().tsb_block_backward(shape, args, floats, int(ctx.has_res), int(causal), stream_ptr(res2.device)), "tsb_block_backward")
-        _native.add_launches(LAUNCHES_BACKWARD - 1)
+                    *grads, _ptr(dres2), wide.data_ptr(), rest.data_ptr(), dx.data_ptr())
+        check(lib().tsb_block_backward(shape, args, floats, int(ctx.has_res), int(causal), stream), "tsb_block_backward")
+        _native.add_launches(LAUNCHES_BACKWARD - 2)
         return (dx, dx if ctx.has_res else None) + (None,) * 13
 
 

@@ -1,5 +1,6 @@
 """The decoder block in one native call, without a GPU: what its autograd function saves and what it takes back, over a stand-in for the library."""
 import ctypes
+import gc
 
 import pytest
 import torch
@@ -13,18 +14,18 @@ PACKED = 4 * 64
 class Library:
     """Entry points that note the addresses they are given."""
 
-    def tsb_block_saved_bytes(self, shape, has_res):
-        return 4096
-
-    def tsb_block_work_bytes(self, shape):
-        return 256
+    def tsb_block_bytes(self, shape, has_res, sizes):
+        sizes[:] = [4096, 8192, 512, 256]
+        return 0
 
     def tsb_block_forward(self, shape, p, f, causal, stream):
         self.forward = list(p)
         return 0
 
+    def tsb_block_backward_down(self, shape, p, stream):
+        return 0
+
     def tsb_block_backward(self, shape, p, f, has_res, causal, stream):
-        self.backward = list(p)
         return 0
 
 
@@ -68,13 +69,17 @@ def _noted(library, has_res=True, given=True, **around):
         params, x, res, (out, res2) = _call(has_res, given)
     seen = {}
 
-    def backward(shape, p, f, has_res, causal, stream):
+    def down(shape, p, stream):
         assert all(v % 16 == 0 for v in p)
-        seen.update(qkv=_at(p[2], PACKED * 128).clone().view(PACKED, 128), gate_up=_at(p[5], 528 * 128).clone().view(528, 128),
-                    down=_at(p[6], 128 * 264).clone().view(128, 264), p=list(p))
+        seen.update(down=_at(p[0], 128 * 264).clone().view(128, 264), first=list(p))
         return 0
 
-    library.tsb_block_backward = backward
+    def backward(shape, p, f, has_res, causal, stream):
+        assert all(v % 16 == 0 for v in p)
+        seen.update(qkv=_at(p[2], PACKED * 128).clone().view(PACKED, 128), gate_up=_at(p[5], 528 * 128).clone().view(528, 128), p=list(p))
+        return 0
+
+    library.tsb_block_backward_down, library.tsb_block_backward = down, backward
     torch.autograd.backward([out, res2], [torch.zeros_like(out), torch.zeros_like(res2)])
     return params, seen
 
@@ -96,13 +101,38 @@ def test_saved_are_whole_stacks(library, has_res, given):
     params, seen = _noted(library, has_res, given, pack=pack, unpack=lambda t: t)
     assert torch.equal(seen["qkv"], torch.cat([p.detach() for p in params[1:4]]))
     assert torch.equal(seen["gate_up"], torch.cat([p.detach() for p in params[6:8]]))
-    assert seen["p"][12] == params[1].main_grad.data_ptr() and seen["p"][15] == params[6].main_grad.data_ptr()
+    assert seen["p"][11] == params[1].main_grad.data_ptr() and seen["p"][14] == params[6].main_grad.data_ptr()
+    assert seen["first"][2] == params[8].main_grad.data_ptr()
     assert library.forward[3] not in (seen["p"][2], seen["p"][5])
 
 
 def test_nothing_is_copied_without_hooks(library):
     params, seen = _noted(library, pack=lambda t: t, unpack=lambda t: t)
-    assert seen["p"][2] == params[1].data_ptr() and seen["p"][5] == params[6].data_ptr() and seen["p"][6] == params[8].data_ptr()
+    assert seen["p"][2] == params[1].data_ptr() and seen["p"][5] == params[6].data_ptr() and seen["first"][0] == params[8].data_ptr()
+
+
+@pytest.mark.parametrize("keep", [False, True])
+def test_widest_activations_are_let_go_halfway(library, keep):
+    """Between the two calls of a backward pass, unless the graph is kept for another one."""
+    _, x, _, (out, _) = _call()
+    size, seen = 8192, []
+
+    def backward(shape, p, f, has_res, causal, stream):
+        gc.collect()
+        seen.append(any(t.dtype is torch.uint8 and t.numel() == size for t in gc.get_objects() if type(t) is torch.Tensor) or _saved(out))
+        return 0
+
+    def _saved(out):
+        try:
+            return any(t.numel() == size for t in out.grad_fn.saved_tensors)
+        except RuntimeError:                              # (let go)
+            return False
+
+    library.tsb_block_backward = backward
+    out.backward(torch.zeros_like(out), retain_graph=keep)
+    if keep:
+        out.backward(torch.zeros_like(out))
+    assert seen == ([True, False] if keep else [False])
 
 
 def test_saved_come_back_off_sixteen_bytes_or_strided(library):
@@ -120,6 +150,6 @@ def test_saved_come_back_off_sixteen_bytes_or_strided(library):
 def test_saved_come_back_as_something_else(library, spoil):
     with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: spoil(t) if t.shape == (128, 264) else t):
         _, _, _, (out, _) = _call()
-    library.tsb_block_backward = None                     # (not reached)
+    library.tsb_block_backward_down = None                # (not reached)
     with pytest.raises(RuntimeError, match="saved tensor"):
         out.backward(torch.zeros_like(out))

@@ -609,6 +609,36 @@ def test_block_under_hooks_on_saved_tensors(dev, kind, has_res):
     _same_blocks(got, want, exact=True)
 
 
+@pytest.mark.parametrize("width,heads,kv,ffn", [(512, 4, 1, 1792), (512, 4, 4, 1024), (512, 8, 8, 1408), (1024, 8, 1, 2048)])
+def test_block_holds_no_more_memory_than_its_modules(dev, width, heads, kv, ffn):
+    """The most that is held during a forward and backward pass over two blocks (32 MB a piece of the stream and more, so that what a
+    few small buffers differ by, or their rounding to 512 bytes, does not count: 1 MB)."""
+    model, arena = _block_model(dev, width, heads, kv, ffn)
+    x, _, dout, dres = _block_inputs(dev, 64, 512, width)
+    x.requires_grad_()
+    most = []
+    for hooked in (False, True):
+        handles = [blk.norm_1.register_forward_hook(lambda *a: None) for blk in model.layers] if hooked else []
+        assert (model.layers[0]._whole(x, None) is None) is hooked
+        for _ in range(2):
+            torch.cuda.synchronize()
+            before = torch.cuda.memory_allocated()
+            torch.cuda.reset_peak_memory_stats()
+            a, r = model.layers[0].forward_fused(x, None)
+            a, r = model.layers[1].forward_fused(a, r)
+            y = model.norm(a, r)[0]
+            del a, r
+            g, = torch.autograd.grad(y, x, dout)
+            torch.cuda.synchronize()
+            peak = torch.cuda.max_memory_allocated() - before
+            del y, g
+        most.append(peak)
+        for h in handles:
+            h.remove()
+    _status_ok()
+    assert most[0] <= most[1] + (1 << 20), most
+
+
 def test_block_runs_its_modules_where_they_are_not_plain(dev):
     from tesseract_b200.nn.modules import Linear
     model, arena = _block_model(dev, 128, 2, 1, 256)
