@@ -21,7 +21,7 @@ _native.register_signatures({
 
 _Shape, _Floats, _Bytes = ctypes.c_longlong * 7, ctypes.c_float * 3, ctypes.c_longlong * 4
 _Fwd, _Down, _Bwd = ctypes.c_longlong * 14, ctypes.c_longlong * 5, ctypes.c_longlong * 19
-LAUNCHES_FORWARD, LAUNCHES_BACKWARD = 9, 18
+LAUNCHES_FORWARD, LAUNCHES_BACKWARD = 9, 17     # backward: eight products, SwiGLU, rotation, three of attention, two per norm
 
 
 def _ptr(t) -> int:

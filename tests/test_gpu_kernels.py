@@ -639,6 +639,27 @@ def test_block_holds_no_more_memory_than_its_modules(dev, width, heads, kv, ffn)
     assert most[0] <= most[1] + (1 << 20), most
 
 
+def test_block_counts_the_launches_of_its_modules(dev):
+    from tesseract_b200 import _native
+    model, arena = _block_model(dev, 256, 2, 1, 688)
+    blk = model.layers[1]
+    x, res, dout, dres = _block_inputs(dev, 2, 40, 256)
+    counts = []
+    for hooked in (False, True):
+        h = blk.norm_1.register_forward_hook(lambda *a: None) if hooked else None
+        arena.zero_grad()
+        x, res = (t.detach().requires_grad_() for t in (x, res))
+        at = [_native.launch_count()]
+        out, stream = blk.forward_fused(x, res)
+        at.append(_native.launch_count())
+        torch.autograd.grad([out, stream], [x, res], [dout, dres])
+        at.append(_native.launch_count())
+        counts.append([b - a for a, b in zip(at[:-1], at[1:])])
+        if h:
+            h.remove()
+    assert counts[0] == counts[1] == [9, 17]
+
+
 def test_block_runs_its_modules_where_they_are_not_plain(dev):
     from tesseract_b200.nn.modules import Linear
     model, arena = _block_model(dev, 128, 2, 1, 256)
