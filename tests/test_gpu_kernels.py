@@ -535,8 +535,8 @@ def _block_model(dev, width, heads, kv, ffn, seed=0):
 @pytest.mark.parametrize("width,heads,kv,ffn,B,S", [(128, 2, 1, 256, 1, 1), (128, 2, 2, 264, 2, 129), (256, 2, 1, 688, 3, 77), (512, 4, 4, 1032, 1, 300),
                                                     (512, 8, 2, 1024, 2, 128)])
 def test_block_in_one_call_gives_what_its_modules_give(dev, width, heads, kv, ffn, B, S):
-    """The same launches, so the same numbers but for dQ, whose parts add up in any order, and the first block's sum of two gradients, rounded once
-    instead of twice; through two blocks each of these moves a value of bf16 by a few last bits (2^-8 each)."""
+    """The same launches, so the same bits, but for the gradient that leaves the first block: it is a sum of two, which the block rounds once (2^-9 of it) and
+    autograd twice; and beyond 256 keys for dQ, whose parts add up in any order, and what depends on it (a last bit of bf16 here and there)."""
     model, arena = _block_model(dev, width, heads, kv, ffn)
     g = torch.Generator(device=dev).manual_seed(S)
     tok, tgt = (torch.randint(0, 96, (B, S), device=dev, generator=g) for _ in range(2))
@@ -549,13 +549,16 @@ def test_block_in_one_call_gives_what_its_modules_give(dev, width, heads, kv, ff
         for _ in range(2):                                     # gradients add up
             loss = model.loss(tok, tgt)
             loss.backward()
-        results.append((float(loss.detach()), [p.main_grad.float().clone() for p in arena.params]))
+        results.append((float(loss.detach()), {n: p.main_grad.clone() for n, p in model.named_parameters()}))
         for h in handles:
             h.remove()
     _status_ok()
     assert results[0][0] == results[1][0]
-    for a, b in zip(results[0][1], results[1][1]):
-        assert float((a - b).norm()) <= 0.02 * float(b.norm()) + 1e-6
+    for n, a in results[0][1].items():
+        if S <= 256 and n != "embed_tokens.weight":
+            assert torch.equal(a, results[1][1][n]), n
+        else:
+            assert _rel_err(a, results[1][1][n].float()) < 5e-3, n
 
 
 def _run_block(blk, arena, x, res, dout, dres, around=contextlib.nullcontext()):
@@ -658,6 +661,66 @@ def test_block_counts_the_launches_of_its_modules(dev):
         if h:
             h.remove()
     assert counts[0] == counts[1] == [9, 17]
+
+
+@pytest.mark.parametrize("width,heads,kv,ffn,B,S", [(128, 2, 1, 264, 2, 1), (256, 2, 2, 688, 1, 129), (512, 4, 1, 1032, 2, 256), (512, 8, 2, 1024, 1, 400)])
+@pytest.mark.parametrize("has_res", [True, False])
+def test_block_against_its_modules_bit_by_bit(dev, width, heads, kv, ffn, B, S, has_res):
+    """As above, with every gradient of one block; what leaves a block without a residual stream behind it is rounded once or twice, 2^-8 at most."""
+    model, arena = _block_model(dev, width, heads, kv, ffn)
+    blk = model.layers[0]
+    x, res, dout, dres = _block_inputs(dev, B, S, width)
+    res = res if has_res else None
+    got = _run_block(blk, arena, x, res, dout, dres)
+    h = blk.norm_1.register_forward_hook(lambda *a: None)
+    want = _run_block(blk, arena, x, res, dout, dres)
+    h.remove()
+    _status_ok()
+    if not has_res:
+        assert _rel_err(got[1].pop(), want[1].pop().float()) < 2 ** -8
+    _same_blocks(got, want, exact=S <= 256)
+
+
+@pytest.mark.parametrize("kind", ["again", "reentrant", "checkpoint", "side", "marker"])
+def test_block_where_autograd_is_used_otherwise(dev, kind):
+    """A graph kept for a second pass, recomputation of either kind, a stream of the program's own, and the marker by which data parallelism hears that a
+    block's gradients are complete: the bits of a plain pass."""
+    from torch.utils.checkpoint import checkpoint
+    from tesseract_b200.parallel.data_parallel import _BucketMarker
+    model, arena = _block_model(dev, 256, 2, 1, 688)
+    blk = model.layers[1]
+    x, res, dout, dres = _block_inputs(dev, 2, 200, 256)
+    want = _run_block(blk, arena, x, res, dout, dres)
+    arena.zero_grad()
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream() if kind == "side" else torch.cuda.current_stream()
+    fired = []
+
+    class Reducer:
+        def _bucket_ready(self, bid):
+            fired.append((bid, {n: p.main_grad.clone() for n, p in blk.named_parameters()}))
+
+    with torch.cuda.stream(side):
+        x, res = (t.detach().clone().requires_grad_() for t in (x, res))
+        ins = [_BucketMarker.apply(t, Reducer(), 3) for t in (x, res)] if kind == "marker" else [x, res]
+        if kind in ("reentrant", "checkpoint"):
+            out, stream = checkpoint(blk.forward_fused, *ins, use_reentrant=kind == "reentrant")
+        else:
+            out, stream = blk.forward_fused(*ins)
+        torch.autograd.backward([out, stream], [dout, dres], retain_graph=kind == "again")
+        if kind == "again":
+            arena.zero_grad()
+            x.grad = res.grad = None
+            torch.autograd.backward([out, stream], [dout, dres])
+    torch.cuda.synchronize()
+    _status_ok()
+    got = ([out.detach(), stream.detach()], [x.grad, res.grad], {n: p.main_grad.clone() for n, p in blk.named_parameters()})
+    _same_blocks(got, want, exact=True)
+    if kind == "marker":
+        assert [bid for bid, _ in fired] == [3, 3] and all(torch.equal(t, got[2][n]) for n, t in fired[0][1].items())
+    if kind == "again":
+        with pytest.raises(RuntimeError):
+            torch.autograd.backward([out, stream], [dout, dres])          # (the graph was given back)
 
 
 def test_block_runs_its_modules_where_they_are_not_plain(dev):
