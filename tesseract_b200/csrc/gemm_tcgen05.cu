@@ -902,6 +902,74 @@ double cta_cost(int M, int N, int K, int bn) {
   return static_cast<double>((tiles + sm_count() - 1) / sm_count()) * bn * (bn == 256 ? (K >= 3072 ? 1.06 : 1.15) : bn == 128 ? 1.33 : bn == 64 ? 2.25 : 4.0);
 }
 
+// Columns of the tiles of one SM, or (pair) the cut for pairs of SMs.
+struct Tiles {
+  int bn;
+  bool pair;
+  PairPlan plan;
+};
+Tiles choose_tiles(int M, int N, int K, int max_ctas) {
+  Tiles t{};
+  const int sms = sm_count();
+  const long long mt = (M + BM - 1) / BM;
+  auto tiles = [&](int b) { return mt * ((N + b - 1) / b); };
+  // largest tile that still gives every SM work; decode-shaped calls (few rows) stream the weight matrix
+  // and want as many CTAs pulling on HBM as possible, so they go down to 32-column tiles
+  if (N >= 256 && tiles(256) >= sms) t.bn = 256;
+  else if (N >= 128 && tiles(128) >= sms) t.bn = 128;
+  else if (N >= 64 && tiles(64) >= sms) t.bn = 64;
+  else if (N >= 128 && tiles(128) * 2 >= sms && mt > 2) t.bn = 128;
+  else t.bn = (N >= 64 && tiles(32) > 2 * sms) ? 64 : 32;
+  // More than one tile of rows, and columns for a wide one: the cheapest kind.
+  if (max_ctas <= 0 && M > 128 && N >= 192) {
+    double best = cta_cost(M, N, K, t.bn);
+    for (const int b : {64, 128, 256})
+      if (const double cost = cta_cost(M, N, K, b); cost < best) {
+        best = cost;
+        t.bn = b;
+      }
+    constexpr int kinds[][2] = {{256, 2}, {256, 1}, {192, 2}, {192, 1}, {128, 1}};
+    for (const auto& kind : kinds) {
+      const PairPlan pl = make_pair_plan(M, N, kind[0], kind[1]);
+      if (const double cost = pair_cost(pl, K); cost < best) {
+        best = cost;
+        t.plan = pl;
+        t.pair = true;
+      }
+    }
+  }
+  return t;
+}
+
+int run_gemm(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc, int a_mn, int b_mn, int out_f32,
+             int accumulate, const Tiles& t, int max_ctas, cudaStream_t s) {
+  CUtensorMap ta, tb;
+  bool ok;
+  if (!a_mn) ok = cached_tmap_2d(&ta, A, M, K, lda * 2, BM, BK);
+  else ok = cached_tmap_2d(&ta, A, K, M, lda * 2, BK, 64);
+  if (!ok) return -3;
+  if (!b_mn) ok = cached_tmap_2d(&tb, B, N, K, ldb * 2, t.pair ? t.plan.n / 2 : t.bn, BK);
+  else ok = cached_tmap_2d(&tb, B, K, N, ldb * 2, BK, 64);
+  if (!ok) return -3;
+  if (t.pair) {
+    if (!a_mn)
+      return b_mn ? launch_pair_out<false, true>(ta, tb, C, M, N, K, ldc, out_f32, accumulate, t.plan, s)
+                  : launch_pair_out<false, false>(ta, tb, C, M, N, K, ldc, out_f32, accumulate, t.plan, s);
+    return b_mn ? launch_pair_out<true, true>(ta, tb, C, M, N, K, ldc, out_f32, accumulate, t.plan, s)
+                : launch_pair_out<true, false>(ta, tb, C, M, N, K, ldc, out_f32, accumulate, t.plan, s);
+  }
+  switch (t.bn) {
+    case 256: return launch_major<256>(ta, tb, C, M, N, K, ldc, a_mn, b_mn, out_f32, accumulate, max_ctas, s);
+    case 128: return launch_major<128>(ta, tb, C, M, N, K, ldc, a_mn, b_mn, out_f32, accumulate, max_ctas, s);
+    case 64: return launch_major<64>(ta, tb, C, M, N, K, ldc, a_mn, b_mn, out_f32, accumulate, max_ctas, s);
+    default: return launch_major<32>(ta, tb, C, M, N, K, ldc, a_mn, b_mn, out_f32, accumulate, max_ctas, s);
+  }
+}
+
+bool gemm_operands_ok(const void* A, const void* B, int M, int N, int K, long long lda, long long ldb) {
+  return M > 0 && N > 0 && K > 0 && !(reinterpret_cast<uintptr_t>(A) & 15) && !(reinterpret_cast<uintptr_t>(B) & 15) && lda % 8 == 0 && ldb % 8 == 0;
+}
+
 }  // namespace
 }  // namespace tsb
 
@@ -918,66 +986,35 @@ TSB_EXPORT int tsb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
                              long long ldb, long long ldc, int a_mn, int b_mn, int out_f32, int accumulate,
                              int block_n, int max_ctas, void* stream) {
   using namespace tsb;
+  if (!gemm_operands_ok(A, B, M, N, K, lda, ldb)) return -2;
+  Tiles t = block_n == 0 ? choose_tiles(M, N, K, max_ctas) : Tiles{block_n, false, {}};
+  if (t.bn == 32 && b_mn) t.bn = 64;  // an N-major B tile is built from 64-column (128-byte) boxes
+  if (t.bn != 32 && t.bn != 64 && t.bn != 128 && t.bn != 256) return -2;
+  return run_gemm(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_f32, accumulate, t, max_ctas, static_cast<cudaStream_t>(stream));
+}
+
+// How tsb_gemm_bf16 (block_n = 0, max_ctas = 0) cuts a product, host array of four: columns of a tile; 1 or 2 of them per tile of a pair of SMs, 0 where
+// the tiles are one SM's; whole tiles; items (whole tiles, and two halves for each of the others).
+TSB_EXPORT int tsb_gemm_bf16_plan(int M, int N, int K, int* out) {
+  using namespace tsb;
   if (M <= 0 || N <= 0 || K <= 0) return -2;
-  if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || (lda % 8) || (ldb % 8))
-    return -2;
-  int bn = block_n;
-  bool pair = false;
-  PairPlan plan{};
-  if (bn == 0) {
-    const int sms = sm_count();
-    const long long mt = (M + BM - 1) / BM;
-    auto tiles = [&](int b) { return mt * ((N + b - 1) / b); };
-    // largest tile that still gives every SM work; decode-shaped calls (few rows) stream the weight matrix
-    // and want as many CTAs pulling on HBM as possible, so they go down to 32-column tiles
-    if (N >= 256 && tiles(256) >= sms) bn = 256;
-    else if (N >= 128 && tiles(128) >= sms) bn = 128;
-    else if (N >= 64 && tiles(64) >= sms) bn = 64;
-    else if (N >= 128 && tiles(128) * 2 >= sms && mt > 2) bn = 128;
-    else bn = (N >= 64 && tiles(32) > 2 * sms) ? 64 : 32;
-    // More than one tile of rows, and columns for a wide one: the cheapest kind.
-    if (max_ctas <= 0 && M > 128 && N >= 192) {
-      double best = cta_cost(M, N, K, bn);
-      for (const int b : {64, 128, 256})
-        if (const double cost = cta_cost(M, N, K, b); cost < best) {
-          best = cost;
-          bn = b;
-        }
-      constexpr int kinds[][2] = {{256, 2}, {256, 1}, {192, 2}, {192, 1}, {128, 1}};
-      for (const auto& kind : kinds) {
-        const PairPlan pl = make_pair_plan(M, N, kind[0], kind[1]);
-        if (const double cost = pair_cost(pl, K); cost < best) {
-          best = cost;
-          plan = pl;
-          pair = true;
-        }
-      }
-    }
-  }
-  if (bn == 32 && b_mn) bn = 64;  // an N-major B tile is built from 64-column (128-byte) boxes
-  if (bn != 32 && bn != 64 && bn != 128 && bn != 256) return -2;
-  CUtensorMap ta, tb;
-  bool ok;
-  if (!a_mn) ok = cached_tmap_2d(&ta, A, M, K, lda * 2, BM, BK);
-  else ok = cached_tmap_2d(&ta, A, K, M, lda * 2, BK, 64);
-  if (!ok) return -3;
-  if (!b_mn) ok = cached_tmap_2d(&tb, B, N, K, ldb * 2, pair ? plan.n / 2 : bn, BK);
-  else ok = cached_tmap_2d(&tb, B, K, N, ldb * 2, BK, 64);
-  if (!ok) return -3;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (pair) {
-    if (!a_mn)
-      return b_mn ? launch_pair_out<false, true>(ta, tb, C, M, N, K, ldc, out_f32, accumulate, plan, s)
-                  : launch_pair_out<false, false>(ta, tb, C, M, N, K, ldc, out_f32, accumulate, plan, s);
-    return b_mn ? launch_pair_out<true, true>(ta, tb, C, M, N, K, ldc, out_f32, accumulate, plan, s)
-                : launch_pair_out<true, false>(ta, tb, C, M, N, K, ldc, out_f32, accumulate, plan, s);
-  }
-  switch (bn) {
-    case 256: return launch_major<256>(ta, tb, C, M, N, K, ldc, a_mn, b_mn, out_f32, accumulate, max_ctas, s);
-    case 128: return launch_major<128>(ta, tb, C, M, N, K, ldc, a_mn, b_mn, out_f32, accumulate, max_ctas, s);
-    case 64: return launch_major<64>(ta, tb, C, M, N, K, ldc, a_mn, b_mn, out_f32, accumulate, max_ctas, s);
-    default: return launch_major<32>(ta, tb, C, M, N, K, ldc, a_mn, b_mn, out_f32, accumulate, max_ctas, s);
-  }
+  const Tiles t = choose_tiles(M, N, K, 0);
+  out[0] = t.pair ? t.plan.n : t.bn;
+  out[1] = t.pair ? t.plan.per : 0;
+  out[2] = t.plan.full;
+  out[3] = t.plan.items;
+  return 0;
+}
+
+// tsb_gemm_bf16 with the kind of tiles given for pairs of SMs, to compare what choose_tiles chooses from: n = 256 or 192 with per = 1 or 2, or 128
+// with 1. More than 128 rows, 192 columns at least.
+TSB_EXPORT int tsb_gemm_bf16_pairs(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc, int a_mn,
+                                   int b_mn, int out_f32, int accumulate, int n, int per, void* stream) {
+  using namespace tsb;
+  if (!gemm_operands_ok(A, B, M, N, K, lda, ldb) || M <= 128 || N < 192) return -2;
+  if (!((n == 256 || n == 192) && (per == 1 || per == 2)) && !(n == 128 && per == 1)) return -2;
+  const Tiles t{0, true, make_pair_plan(M, N, n, per)};
+  return run_gemm(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_f32, accumulate, t, 0, static_cast<cudaStream_t>(stream));
 }
 
 // Grouped GEMM for mixture-of-experts layers; `offsets` (int32 [groups + 1], multiples of 128) stays on the device.

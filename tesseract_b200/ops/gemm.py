@@ -62,6 +62,21 @@ _native.register_signatures({
 })
 
 
+_native.register_signatures({
+    "tsb_gemm_bf16_plan": [_native.I, _native.I, _native.I, _native.P],
+    "tsb_gemm_bf16_pairs": _native._SIGNATURES["tsb_gemm_bf16"],
+})
+
+
+def gemm_plan(M: int, N: int, K: int) -> tuple:
+    """How ``gemm_bf16`` cuts a product on the current device: (columns of a tile, tiles' halves per pair of SMs or 0 where they are one SM's,
+    whole tiles, items)."""
+    import ctypes
+    out = (ctypes.c_int * 4)()
+    _native.check(_native.lib().tsb_gemm_bf16_plan(M, N, K, out), "tsb_gemm_bf16_plan")
+    return tuple(out)
+
+
 def plan_decode_gemm(M: int, N: int, K: int, sm_count: int = 148, mode: str = "cluster"):
     """How a decode-shaped product x [M, K] @ w [N, K]^T is run: ``("cluster", S)`` -- S K-slices per output tile,
     reduced through the shared memory of a thread-block cluster; ``("plain", 0)`` -- the persistent GEMM;

@@ -70,7 +70,7 @@ def test_gemm_block_sizes_and_fp32_accumulate(dev, block_n):
 
 
 def test_gemm_persistent_many_tiles(dev):
-    """More tiles than SMs: exercises the smem ring / TMEM double-buffer phase flips."""
+    """More tiles than SMs: exercises the smem ring / TMEM double-buffer phase flips (on pairs of SMs; tiles of one SM: see below)."""
     from tesseract_b200.ops import gemm_bf16
     M, N, K = 4096, 4096, 1024
     A = torch.randn(M, K, device=dev).bfloat16() * 0.1
@@ -473,9 +473,9 @@ def test_tiny_llama_train_step_matches_cpu(dev):
     assert worst < 8e-2, worst
 
 
-@pytest.mark.parametrize("M,N,K,pad", [(4864, 4096, 64, 0), (4872, 4104, 520, 0), (9000, 2312, 136, 0),      # 128 x 256 tiles; from here on pairs
+@pytest.mark.parametrize("M,N,K,pad", [(4864, 4096, 64, 0), (4872, 4104, 520, 0), (9000, 2312, 136, 0),      # pairs: halves of 192, and of 256
                                        (4864, 4096, 960, 0), (4872, 4104, 1032, 0), (9000, 2312, 1000, 3), (4864, 4096, 12288, 0),
-                                       (4864, 4096, 12352, 0)])                                  # the last: pairs for both operands along M and N
+                                       (4864, 4096, 12352, 0)])                                  # the last two: whole tiles of 256 x 384
 @pytest.mark.parametrize("a_mn", [False, True])
 @pytest.mark.parametrize("b_mn", [False, True])
 @pytest.mark.parametrize("out,accumulate", [(torch.bfloat16, False), (torch.bfloat16, True), (torch.float32, True)])
@@ -497,17 +497,21 @@ def test_gemm_tiles_of_two_sms(dev, M, N, K, pad, a_mn, b_mn, out, accumulate):
     assert torch.equal(rows[:, N:], beside)
 
 
-@pytest.mark.parametrize("M,N,K,pad", [(3000, 6392, 6152, 0), (3000, 6392, 6152, 3),   # tiles of 256 x 512, the rest as halves, some beyond N
-                                       (2600, 2048, 8200, 0),                          # 256 x 384 whole
-                                       (3000, 2048, 2056, 0), (1072, 1152, 3264, 0),   # halves of 192, of 128
-                                       (2600, 12104, 72, 0)])                          # of 256, two blocks of K
+@pytest.mark.parametrize("M,N,K,pad,cut", [(3000, 4104, 6152, 0, (256, 2, 74, 142)), (3000, 4104, 6152, 3, (256, 2, 74, 142)),     # whole tiles, then halves, some beyond N
+                                           (1800, 6392, 6152, 0, (256, 2, 74, 134)), (3000, 5384, 6152, 0, (192, 2, 148, 212)),
+                                           (3000, 6392, 6152, 0, (192, 2, 204, 204)), (3000, 6392, 6152, 3, (192, 2, 204, 204)),
+                                           (2600, 2048, 8200, 0, (192, 2, 66, 66)),                                                # whole tiles only
+                                           (3000, 2048, 2056, 0, (192, 1, 132, 132)), (1072, 1152, 3264, 0, (128, 1, 45, 45)),     # halves only
+                                           (2600, 12104, 72, 0, (256, 1, 528, 528))])                                              # two blocks of K
 @pytest.mark.parametrize("a_mn", [False, True])
 @pytest.mark.parametrize("b_mn", [False, True])
 @pytest.mark.parametrize("out,accumulate", [(torch.bfloat16, False), (torch.bfloat16, True), (torch.float32, False)])
-def test_gemm_kinds_of_tiles(dev, M, N, K, pad, a_mn, b_mn, out, accumulate):
-    """Every kind of tile of two SMs at its edges, stored by TMA or (rows off 16 bytes) directly. Bounds as above; a wrong column or row of
-    a tile would stand out by the size of the result."""
-    from tesseract_b200.ops.gemm import gemm_bf16
+def test_gemm_kinds_of_tiles(dev, M, N, K, pad, cut, a_mn, b_mn, out, accumulate):
+    """Every kind of tile of two SMs that the rule chooses (``cut``, on 148 SMs) at its edges, stored by TMA or (rows off 16 bytes) directly. Bounds as
+    above; a wrong column or row of a tile would stand out by the size of the result."""
+    from tesseract_b200.ops.gemm import gemm_bf16, gemm_plan
+    if torch.cuda.get_device_properties(dev).multi_processor_count == 148:
+        assert gemm_plan(M, N, K) == cut
     g = torch.Generator(device=dev).manual_seed(M + N + K)
     a = torch.randn(*((K, M) if a_mn else (M, K)), device=dev, generator=g).bfloat16()
     b = torch.randn(*((K, N) if b_mn else (N, K)), device=dev, generator=g).bfloat16()
@@ -521,6 +525,68 @@ def test_gemm_kinds_of_tiles(dev, M, N, K, pad, a_mn, b_mn, out, accumulate):
     # a value's error: half a step of bf16, 2^-9 of the largest, or what fp32 sums of this depth leave
     assert float((c.double() - ref).abs().max()) <= float(ref.abs().max()) * (2.0 ** -8 if out == torch.bfloat16 else 1e-4)
     assert torch.equal(rows[:, N:], beside)
+
+
+def _gemm_layouts(dev, M, N, K, pad, run, pairs_of=((torch.bfloat16, False), (torch.bfloat16, True), (torch.float32, False), (torch.float32, True))):
+    """All layouts of the operands and forms of the result of one size, by ``run(a, b, c, a_mn, b_mn, accumulate)``; bounds as above."""
+    g = torch.Generator(device=dev).manual_seed(M + N + K)
+    a, b = torch.randn(M, K, device=dev, generator=g).bfloat16(), torch.randn(N, K, device=dev, generator=g).bfloat16()
+    product = a.double() @ b.double().t()
+    for out, accumulate in pairs_of:
+        rows = torch.randn(M, N + pad, device=dev, generator=g).to(out)
+        ref = product + (rows[:, :N].double() if accumulate else 0)
+        for a_mn in (False, True):
+            for b_mn in (False, True):
+                got = rows.clone()
+                run(a.t().contiguous() if a_mn else a, b.t().contiguous() if b_mn else b, got[:, :N], a_mn, b_mn, accumulate)
+                torch.cuda.synchronize()
+                _status_ok()
+                what = (out, accumulate, a_mn, b_mn)
+                c = got[:, :N].double()
+                assert float((c - ref).norm() / ref.norm()) < (3e-3 if out == torch.bfloat16 else 1e-4), what
+                assert float((c - ref).abs().max()) <= float(ref.abs().max()) * (2.0 ** -8 if out == torch.bfloat16 else 1e-4), what
+                assert torch.equal(got[:, N:], rows[:, N:]), what
+
+
+@pytest.mark.parametrize("n,per", [(256, 2), (192, 2), (256, 1), (192, 1), (128, 1)])
+@pytest.mark.parametrize("M,wide,K,pad", [(2248, 9, 264, 0), (2248, 9, 264, 3), (5000, 8, 8, 0), (5000, 8, 72, 0), (5000, 8, 584, 0)])
+def test_gemm_each_kind_of_tiles(dev, n, per, M, wide, K, pad):
+    """Each kind by itself, at sizes that have all of it: a last column of tiles with one half (so that the next one starts on the other accumulator),
+    several tiles per pair, the rest of a round as halves, some beyond N, and one to ten blocks of K in rings of four and of six."""
+    from tesseract_b200 import _native
+    N = (wide - 1) * per * n + n - 56
+    pairs, tiles = torch.cuda.get_device_properties(dev).multi_processor_count // 2, -(-M // 256) * wide
+    assert pairs != 74 or (tiles > pairs and 0 < 2 * (tiles % pairs) <= pairs)
+
+    def run(a, b, c, a_mn, b_mn, accumulate):
+        _native.check(_native.lib().tsb_gemm_bf16_pairs(a.data_ptr(), b.data_ptr(), c.data_ptr(), M, N, K, a.stride(0), b.stride(0), c.stride(0), int(a_mn),
+                                                        int(b_mn), int(c.dtype == torch.float32), int(accumulate), n, per,
+                                                        _native.stream_ptr(a.device)), "tsb_gemm_bf16_pairs")
+    _gemm_layouts(dev, M, N, K, pad, run)
+
+
+def test_gemm_kinds_that_there_are_not(dev):
+    from tesseract_b200 import _native
+    a = torch.zeros(512, 64, device=dev, dtype=torch.bfloat16)
+    c = torch.zeros(512, 512, device=dev, dtype=torch.bfloat16)
+    call = lambda M, N, n, per: _native.lib().tsb_gemm_bf16_pairs(a.data_ptr(), a.data_ptr(), c.data_ptr(), M, N, 64, 64, 64, 512, 0, 0, 0, 0, n, per,
+                                                                  _native.stream_ptr(a.device))
+    assert all(call(*w) == -2 for w in ((512, 512, 128, 2), (512, 512, 64, 1), (512, 512, 256, 3), (512, 512, 256, 0), (128, 512, 256, 1), (512, 184, 256, 1)))
+    assert call(512, 512, 256, 2) == 0
+    torch.cuda.synchronize()
+    _status_ok()
+
+
+@pytest.mark.parametrize("bn", [64, 128, 256])
+@pytest.mark.parametrize("ctas", [0, 37])
+@pytest.mark.parametrize("K", [72, 1000])
+def test_gemm_tiles_of_one_sm_many_per_cta(dev, bn, ctas, K):
+    """Three and twelve tiles per CTA (the phases of ring and accumulators flip), ragged ends of all three sizes."""
+    from tesseract_b200.ops.gemm import gemm_bf16
+    M, N = 2616, 20 * bn + 40
+    _gemm_layouts(dev, M, N, K, 0, lambda a, b, c, a_mn, b_mn, accumulate: gemm_bf16(a, b, a_mn=a_mn, b_mn=b_mn, out=c, accumulate=accumulate, block_n=bn,
+                                                                                    max_ctas=ctas),
+                  ((torch.bfloat16, False), (torch.float32, True)))
 
 
 def _block_model(dev, width, heads, kv, ffn, seed=0):
