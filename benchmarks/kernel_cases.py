@@ -98,6 +98,48 @@ def case_gemm(b: Bench):
     report("gemm", ms, flops=2.0 * M * N * K, shape=[M, N, K])
 
 
+def case_gemm_kinds(b: Bench):
+    """What chooses the tiles of a product against all that it chooses from: products of training and prompts, every kind of tile in turn, each repeated
+    for 40 ms (so that the power limit is part of it), best of two. One line per product, and one with what the choice costs over all of them."""
+    from tesseract_b200 import _native
+    from tesseract_b200.ops.gemm import gemm_bf16, gemm_plan
+
+    def sustained(fn):
+        fn()
+        torch.cuda.synchronize()
+        best, n = 1e9, 2
+        for _ in range(3):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            for _ in range(n):
+                fn()
+            e1.record()
+            torch.cuda.synchronize()
+            t = e0.elapsed_time(e1) / n
+            best, n = min(best, t) if n > 2 else best, max(3, int(40.0 / t))
+        return best * 1e3
+
+    lost = []
+    for N, K in ((6144, 4096), (4096, 4096), (28672, 4096), (4096, 14336), (32000, 4096), (3072, 2048), (2048, 2048), (16384, 2048), (2048, 8192), (768, 256),
+                 (1376, 256), (1288, 1000)):
+        for M in (192, 512, 1024, 2048, 3003, 4096, 8192, 17000):
+            a, w = b.randn(M, K), b.randn(N, K, scale=0.02)
+            out = torch.empty(M, N, device=b.dev, dtype=torch.bfloat16)
+            s = _native.stream_ptr(b.dev)
+            pairs = lambda n, per: _native.check(_native.lib().tsb_gemm_bf16_pairs(a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, K, K, N, 0, 0, 0, 0, n,
+                                                                                   per, s), "pairs")
+            times = {f"{n}x{per}": sustained(lambda: pairs(n, per)) for n, per in ((256, 2), (256, 1), (192, 2), (192, 1), (128, 1))}
+            times.update({str(bn): sustained(lambda: gemm_bf16(a, w, out=out, block_n=bn)) for bn in (32, 64, 128, 256)})
+            n, per, _, _ = gemm_plan(M, N, K)
+            chosen, best = f"{n}x{per}" if per else str(n), min(times, key=times.get)
+            lost.append(times[chosen] / times[best])
+            print(json.dumps({"case": "gemm_kinds", "shape": [M, N, K], "chosen": chosen, "best": best, "chosen_over_best": round(lost[-1], 3),
+                              "us": {k: round(t, 1) for k, t in times.items()}}), flush=True)
+    lost.sort()
+    print(json.dumps({"case": "gemm_kinds", "products": len(lost), "mean_over_best": round(sum(lost) / len(lost), 4), "median": round(lost[len(lost) // 2], 3),
+                      "p90": round(lost[int(0.9 * len(lost))], 3), "worst": round(lost[-1], 3)}), flush=True)
+
+
 def case_gemm_wgrad(b: Bench):
     from tesseract_b200.ops import gemm_bf16
     T, N, K = 16384, 4096, 4096
@@ -765,7 +807,7 @@ def case_gelu_glu(b: Bench):
     report("gelu_glu", b.time(lambda: ops.gelu_glu(x)), bytes_=x.numel() * 2 * 1.5, shape=list(x.shape))
 
 
-CASES = {"gemm": case_gemm, "gemm_fp8": case_gemm_fp8, "gemm_fp8_pertensor": case_gemm_fp8_pertensor, "decode_gemm": case_decode_gemm, "gemm_wgrad": case_gemm_wgrad, "grouped_gemm": case_grouped_gemm,
+CASES = {"gemm": case_gemm, "gemm_fp8": case_gemm_fp8, "gemm_fp8_pertensor": case_gemm_fp8_pertensor, "decode_gemm": case_decode_gemm, "gemm_wgrad": case_gemm_wgrad, "gemm_kinds": case_gemm_kinds, "grouped_gemm": case_grouped_gemm,
          "flash_fwd": case_flash_fwd, "flash_bwd": case_flash_bwd, "decode": case_decode,
          "decode_int8": case_decode_int8, "rmsnorm": case_rmsnorm, "swiglu": case_swiglu, "swiglu_bwd": case_swiglu_bwd, "adam": case_adam,
          "ce_stats": case_ce, "selective_scan": case_scan, "gemv_w8": case_gemv, "gemm_rs_emul": case_gemm_rs_emul,

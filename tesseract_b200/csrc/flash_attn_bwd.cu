@@ -22,8 +22,10 @@
 //                   5500 clocks a step of all SMs), of which bulk reductions reach less (16384 tokens, 32 / 8 heads, causal: 6.4
 //                   against 6.6 ms).
 //   warp 12         TMA producer       warp 13   allocates TMEM, issues the MMAs      (warps 14, 15 only give their registers)
-// Order of the MMAs of step i: dP_i, dV_i, S_{i+1}, dK_i, dQ_i. dP_i needs no probabilities and S_{i+1} no gradients, so that
-// P of step i + 1 is formed while dK_i, dQ_i and dP_{i+1} run, and dS_i while dV_i and S_{i+1} do.
+// Order of the MMAs of step i. Heads of 128, whose dQ lies over dP: dP_i, dV_i, S_{i+1}, dK_i, dQ_i. dP_i needs no probabilities and S_{i+1} no
+// gradients, so that P of step i + 1 is formed while dK_i, dQ_i and dP_{i+1} run, and dS_i while dV_i and S_{i+1} do. Heads of 64, whose dQ has columns
+// of its own: dV_i, S_{i+1}, dK_i, dP_{i+1}, dQ_i (dP_0 in front of all). There dP_{i+1} being ready says nothing about dQ_i, so that of dS_{i+1} in
+// shared memory only the compute warps' wait for dQ_i keeps dS_i from being overwritten under it.
 //
 // Measured, all of the backward pass (32 / 8 heads of 128, causal), L2 flushed: 2 x 4096 tokens 0.83 ms, 16384 tokens 6.2 ms (885 TFLOP/s; 0.87
 // and 6.4 with one lane's issue loops), against 1.89 and 13.6 for four warps that went through scores, P, dS and dQ of a tile one after another;
@@ -374,7 +376,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
       for (int e = 0; e < 8; ++e) dl[e] = reinterpret_cast<const float4*>(delta)[e];
       here = mbar_wait(&dp_full, ph, &cta_abort, p.status);
-      // dK and dQ of the step before have read dS (its first pass finds the barrier open)
+      // dQ of the step before has read dS in shared memory (its first pass finds the barrier open). Heads of 64 have no other wait for that: the dP
+      // waited for above was issued in front of that dQ.
       here = here && mbar_wait(&dq_full, ph ^ 1u, &cta_abort, p.status);
       if (!__all_sync(0xffffffffu, here ? 1 : 0)) { ok = false; break; }
       tc_fence_after();
