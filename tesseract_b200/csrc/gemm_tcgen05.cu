@@ -884,17 +884,20 @@ PairPlan make_pair_plan(int M, int N, int n, int per) {
 }
 
 // What a product takes with tiles of a kind, up to a factor that they share: the tiles that one SM (or pair) works on in turn, times the
-// columns of a tile, times how much slower a column is than in the widest ones. The figures are times of 35 products of training and
-// prompts (64 - 18944 rows, depths 128 - 28672), all kinds of tiles in turn. Deep products want whole tiles of 256 x 512 (8192 x 4096 x 28672:
-// 1393 us against 1475 for halves by themselves; 4096 deep the same), shallow ones halves, whose stores start earlier (3003 x 16384 x 2048: 163
-// against 166). Widths of 192 fit where 256 would leave most of a round empty (3003 x 2048 x 8192: 72 against 93). Tiles of one SM remain for
-// up to 128 rows, for few tiles (296 x 2176 x 5120: 64 columns 18.5, pairs 23.8 at best) and where the last pair of row tiles would be half
-// empty (528 x 44384 x 3264: 142 against 166).
+// columns of a tile, times how much slower a column is than in the widest ones. The factors are fitted to the times of all kinds at 351 products of training
+// and prompts (forward and both gradients; 136 - 17000 rows, 256 - 32000 columns, depths 136 - 32000): what is chosen takes 2.4 % more than the best kind in
+// the mean, nothing in the median, at most 27 % (launches of 7 us, and gradients of 512 - 1024 rows; `kernel_cases.py --case gemm_kinds` has the
+// forward ones). Deep products want whole tiles of 256 x 512 (input gradient 4096 x 4096 x 28672: 744 us against 759 for halves by themselves), others halves,
+// whose stores start earlier (all in turn, 60 ms at a time: weight gradients 128256 x 4096 x 4096 2878 against 3792, 4096 x 14336 x 4096 339 against 422,
+// forward 8192 x 28672 x 4096 1291 against 1424). Widths of 192 fit where 256 would leave most of a round empty (3003 x 2048 x 8192: 72 against 93), but a
+// column of theirs costs more, of whole tiles too (8192 x 6144 x 4096: 327 against 301 for halves of 256; input gradient 1024 x 14336 x 4096
+// 115 against 106). Tiles of one SM remain for up to 128 rows, for few tiles
+// (296 x 2176 x 5120: 64 columns 18.5, pairs 23.8 at best) and where the last pair of row tiles would be half empty (528 x 44384 x 3264: 142 against 166).
 double pair_cost(const PairPlan& pl, int K) {
   const int pairs = sm_count() / 2, halves = pl.items - pl.full;
   const int rounds = (pl.full + pairs - 1) / pairs * pl.per + (halves > 0 ? 1 : 0);
-  const double slow = (pl.per == 2 ? 1.0 : K >= 6144 ? 1.05 : K >= 3072 ? 1.0 : 0.95) *
-                      (pl.n == 256 ? 1.0 : pl.n == 128 ? 1.25 : pl.per == 2 ? 1.04 : 1.08);
+  const double slow = (pl.per == 2 ? 1.0 : K >= 6144 ? 1.05 : K >= 3072 ? 0.98 : 0.95) *
+                      (pl.n == 256 ? 1.0 : pl.n == 128 ? 1.25 : 1.08);
   return rounds * pl.n * slow;
 }
 double cta_cost(int M, int N, int K, int bn) {
