@@ -157,58 +157,43 @@ TSB_EXPORT int tsb_block_forward(const long long* shape, const long long* p, con
   return product(k.act, p[7], out, W, F);
 }
 
-namespace tsb {
-namespace {
-
-int product_input(const void* dy, long long weight, void* d, int rows, int outs, int ins, long long ldd, void* stream) {      // d = dy W
-  return tsb_gemm_bf16(dy, ptr(weight), d, rows, ins, outs, outs, ins, ldd, 0, 1, 0, 0, 0, 0, stream);
-}
-int product_weight(const void* dy, const void* x, long long d, int rows, int outs, int ins, void* stream) {                   // dW += dy^T x
-  return tsb_gemm_bf16(dy, x, ptr(d), outs, ins, rows, outs, ins, ins, 1, 1, 0, 1, 0, 0, stream);
-}
-
-}  // namespace
-}  // namespace tsb
-
-// Gradients of the above, first part: from the block's output to gate and up. What `mid` holds is not needed after it.
-// p: down weight, mid, gradient of down (added to; bf16), dout, wide.
-TSB_EXPORT int tsb_block_backward_down(const long long* shape, const long long* p, void* stream) {
+// Gradients of the above, in two parts: 1, from the block's output to gate and up, after which what `mid` holds is not needed, then 2, the rest.
+// p: x (where there was no res; else unused), norm_1, qkv, o, norm_2, gate and up, down (weights), cos, sin, saved, mid, res2, gradients of norm_1, qkv, o,
+// norm_2, gate and up, down (added to; bf16), dout, dres2 (0: none), wide (kept between the parts), rest, dx (of x and of res). Part 1 touches
+// neither rest nor dx, part 2 neither mid nor dout. f: as forward.
+TSB_EXPORT int tsb_block_backward(const long long* shape, const long long* p, const float* f, int has_res, int causal, int part, void* stream) {
   using namespace tsb;
   const BlockShape s = shape_of(shape);
-  if (!s.ok()) return -2;
-  const Saved k(s, nullptr, ptr(p[1]), false);
-  const int T = static_cast<int>(s.rows()), W = s.W, F = s.F;
-  const void* dout = ptr(p[3]);
-  void* dgu = ptr(p[4]);
-  int rc = product_input(dout, p[0], dgu, T, W, F, 2LL * F, stream);
-  if (rc) return rc;
-  if ((rc = product_weight(dout, k.act, p[2], T, W, F, stream))) return rc;
-  return tsb_swiglu_bwd_rows(dgu, 2LL * F, k.gu, dgu, T, F, kBf16, stream);
-}
-
-// The rest. p: x (where there was no res; else unused), norm_1, qkv, o, norm_2, gate and up (weights), cos, sin, saved, res2, gradients of norm_1,
-// qkv, o, norm_2, gate and up (added to; bf16), dres2 (0: none), wide (as the first part left it), rest, dx (of x and of res). f: as forward.
-TSB_EXPORT int tsb_block_backward(const long long* shape, const long long* p, const float* f, int has_res, int causal, void* stream) {
-  using namespace tsb;
-  const BlockShape s = shape_of(shape);
-  if (!s.ok()) return -2;
-  const Saved k(s, ptr(p[8]), nullptr, has_res != 0);
-  const Work w(s, ptr(p[16]), ptr(p[17]));
+  if (!s.ok() || (part != 1 && part != 2)) return -2;
+  const Saved k(s, ptr(p[9]), ptr(p[10]), has_res != 0);
+  const Work w(s, ptr(p[20]), ptr(p[21]));
   const int T = static_cast<int>(s.rows()), N = static_cast<int>(s.packed()), W = s.W, F = s.F, D = s.D;
+  auto input = [&](const void* dy, long long weight, void* d, int outs, int ins, long long ldd) {         // d = dy W
+    return tsb_gemm_bf16(dy, ptr(weight), d, T, ins, outs, outs, ins, ldd, 0, 1, 0, 0, 0, 0, stream);
+  };
+  auto weight = [&](const void* dy, const void* x, long long d, int outs, int ins) {                      // dW += dy^T x
+    return tsb_gemm_bf16(dy, x, ptr(d), outs, ins, T, outs, ins, ins, 1, 1, 0, 1, 0, 0, stream);
+  };
+  int rc = 0;
+  if (part == 1) {
+    const void* dout = ptr(p[18]);
+    if ((rc = input(dout, p[6], w.wide, W, F, 2LL * F))) return rc;
+    if ((rc = weight(dout, k.act, p[17], W, F))) return rc;
+    return tsb_swiglu_bwd_rows(w.wide, 2LL * F, k.gu, w.wide, T, F, kBf16, stream);
+  }
   const long long row = N, seq = static_cast<long long>(s.S) * N, hd = static_cast<long long>(s.H) * D, vd = hd + static_cast<long long>(s.Hkv) * D;
-  void *dx = ptr(p[18]), *dh2 = dx, *d_o = dx, *dh1 = w.wide;
-  int rc = product_input(w.wide, p[5], dh2, T, 2 * F, W, W, stream);
-  if (rc) return rc;
-  if ((rc = product_weight(w.wide, k.h2, p[14], T, 2 * F, W, stream))) return rc;
-  if ((rc = tsb_rmsnorm_bwd(dh2, ptr(p[9]), ptr(p[4]), k.rstd2, ptr(p[15]), w.da, ptr(p[13]), w.partial, T, W, 1, kBf16, stream))) return rc;
-  if ((rc = product_input(w.da, p[3], d_o, T, W, W, W, stream))) return rc;
-  if ((rc = product_weight(w.da, k.o, p[12], T, W, W, stream))) return rc;
+  void *dx = ptr(p[22]), *dh2 = dx, *d_o = dx, *dh1 = w.wide;
+  if ((rc = input(w.wide, p[5], dh2, 2 * F, W, W))) return rc;
+  if ((rc = weight(w.wide, k.h2, p[16], 2 * F, W))) return rc;
+  if ((rc = tsb_rmsnorm_bwd(dh2, ptr(p[11]), ptr(p[4]), k.rstd2, ptr(p[19]), w.da, ptr(p[15]), w.partial, T, W, 1, kBf16, stream))) return rc;
+  if ((rc = input(w.da, p[3], d_o, W, W, W))) return rc;
+  if ((rc = weight(w.da, k.o, p[14], W, W))) return rc;
   rc = tsb_flash_bwd(d_o, k.qkv, k.qkv + hd * 2, k.qkv + vd * 2, k.o, k.lse, w.dqkv, w.dqkv + hd * 2, w.dqkv + vd * 2, w.wide, s.B, s.S, s.S,
                      s.H, s.Hkv, D, seq, row, D, seq, row, D, seq, row, D, seq, row, D, f[2], causal, stream);
   if (rc) return rc;
-  rc = tsb_rope_qkv(w.dqkv, ptr<float>(p[6]), ptr<float>(p[7]), nullptr, T, s.S, 0, s.H + s.Hkv, s.H + 2 * s.Hkv, D, -1.f, kBf16, stream);
+  rc = tsb_rope_qkv(w.dqkv, ptr<float>(p[7]), ptr<float>(p[8]), nullptr, T, s.S, 0, s.H + s.Hkv, s.H + 2 * s.Hkv, D, -1.f, kBf16, stream);
   if (rc) return rc;
-  if ((rc = product_input(w.dqkv, p[2], dh1, T, N, W, W, stream))) return rc;
-  if ((rc = product_weight(w.dqkv, k.h1, p[11], T, N, W, stream))) return rc;
-  return tsb_rmsnorm_bwd(dh1, has_res ? k.res1 : ptr(p[0]), ptr(p[1]), k.rstd1, w.da, dx, ptr(p[10]), w.partial, T, W, 1, kBf16, stream);
+  if ((rc = input(w.dqkv, p[2], dh1, N, W, W))) return rc;
+  if ((rc = weight(w.dqkv, k.h1, p[13], N, W))) return rc;
+  return tsb_rmsnorm_bwd(dh1, has_res ? k.res1 : ptr(p[0]), ptr(p[1]), k.rstd1, w.da, dx, ptr(p[12]), w.partial, T, W, 1, kBf16, stream);
 }

@@ -69,8 +69,8 @@ class ParamArena:
         g = self.grad
         size = g.numel() * g.element_size()
         # (kernels go to the current device: a buffer on another one, or a checkout without a built library, is torch's to clear)
-        if (g.is_cuda and size % 32 == 0 and g.data_ptr() % 32 == 0 and g.device.index == torch.cuda.current_device() and _native.available()
-                and hasattr(lib(), "tsb_zero")):
+        if (g.is_cuda and size % 32 == 0 and g.data_ptr() % 32 == 0 and g.device.index == torch.cuda.current_device()
+                and (_native._lib is not None or _native.available()) and hasattr(lib(), "tsb_zero")):
             check(lib().tsb_zero(g.data_ptr(), size, stream_ptr(g.device)), "tsb_zero")
         else:
             g.zero_()

@@ -670,7 +670,7 @@ def _same_blocks(a, b, exact):
 @pytest.mark.parametrize("kind", ["copy", "host", "pinned", "off"])
 @pytest.mark.parametrize("has_res", [True, False])
 def test_block_under_hooks_on_saved_tensors(dev, kind, has_res):
-    """What is saved may come back somewhere else (activations kept on the host): weights with all their rows, from any address on."""
+    """What is saved may come back somewhere else (activations kept on the host), at any address; the weights' rows are all there."""
     model, arena = _block_model(dev, 256, 2, 1, 688)
     blk = model.layers[1]
     x, res, dout, dres = _block_inputs(dev, 2, 150, 256)

@@ -123,6 +123,7 @@ def test_gradients_are_cleared_on_their_own_device(monkeypatch, device, built, s
     a.grad, a.params = grad, []
     monkeypatch.setattr(module, "lib", lib)
     monkeypatch.setattr(module, "stream_ptr", lambda d: 0)
+    monkeypatch.setattr("tesseract_b200._native._lib", None)
     monkeypatch.setattr("tesseract_b200._native.available", lambda: built)
     monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
     a.zero_grad()
