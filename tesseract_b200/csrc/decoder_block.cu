@@ -1,9 +1,9 @@
-// One pre-norm decoder block, forward and backward, as one call each: the launches that ops.rms_norm, linear, rope_qkv, flash_attention_packed
+// One pre-norm decoder block, forward in one call and backward in two: the launches that ops.rms_norm, linear, rope_qkv, flash_attention_packed
 // and swiglu make one by one, in the same order, over buffers that are laid out here.
 //
 // What bounds a training step of a small model is the host: a block is 9 launches forward and 17 backward, and issuing each through Python,
 // autograd and ctypes took 29 us of host time, where the GPU worked 2 - 10 (4 layers of width 256, 4 x 128 tokens: 4.2 ms a step, 0.65 of them
-// kernels). From here: 1.53 ms.
+// kernels). From here: 1.59 ms.
 #include "common.cuh"
 
 #include <algorithm>

@@ -622,7 +622,10 @@ double plan_family(int M, int N, int kb, bool fp8, int fixed_bn, int rb, int* bn
       const int ctas = tiles * s * row_ctas;
       if (ctas > cap) continue;
       const double useful = static_cast<double>(N) / (static_cast<double>(tiles) * bn);
-      // at equal CTA counts the plan with fewer K steps per CTA wins (a step costs about the same whatever its width)
+      // at equal CTA counts the plan with fewer K steps per CTA wins. (This and the factors below were measured with issue loops of one lane, where a step
+      // cost about the same whatever its width; they have not been fitted again to the loops there are now. Planned against the best of a sweep,
+      // us, launches behind one another: 6144 x 4096 and 4096 x 14336 within 2 % at 8 and 64 rows; 3072 x 2048 7.9 / 6.7 and 8.6 / 8.5; 2048 x 8192
+      // 15.2 / 11.3 and 15.7 / 12.9, the best being 160 - 224 columns and 8 slices.)
       double score = static_cast<double>(ctas) * useful - 0.02 * ((kb + s - 1) / s);
       if (kb / s < 16) score *= 0.85;
       if (s == 8) score *= 0.9;

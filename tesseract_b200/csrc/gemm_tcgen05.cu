@@ -397,15 +397,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 //                 bytes moved through the L2 and shared memory cost it. No accumulator is left to work on during the stores; instead the halves of a tile run
 //                 apart by as many blocks of K as the ring holds, at its end (the first is stored while the second catches up) and at its start.
 //   halves        256 x n, one accumulator after the other: the rest of the tiles where that is at most a round of halves, and products
-//                 that have few tiles or little depth.
+//                 that have few tiles or are less than 6144 deep (the first half's stores start earlier).
 // Rows leave through shared memory and TMA; an accumulated product reads what it adds to while its products are formed.
 //   every CTA   warp 0 loads its halves of A and B; the bytes are counted on the first CTA's barrier. Warps 2-5 store its rows.
 //   first CTA   warp 1 issues the MMAs; its commits arrive in both CTAs.
-// Sustained under the power limit, against tiles of 256 x 256 only, issued by one lane's loop and stored from registers, in turn (us):
-//   forward          8192 x 28672 x 4096 1489 -> 1361    8192 x 4096 x 14336 790 -> 674     3003 x 2048 x 8192 106 -> 86
-//   input gradient   8192 x 4096 x 28672 1575 -> 1362    8192 x 14336 x 4096 796 -> 711     3003 x 2048 x 16384 208 -> 171
-//   weight gradient  28672 x 4096 x 8192 1690 -> 1517    128256 x 4096 x 4096 3788 -> 3502  16384 x 2048 x 3003 179 -> 162
-// (1250 - 1430 TFLOP/s for the large ones.)
+// Sustained under the power limit, against tiles of 256 x 256 only, issued by one lane's loop and stored from registers (us):
+//   forward          8192 x 28672 x 4096 1489 -> 1327    8192 x 4096 x 14336 790 -> 669     3003 x 2048 x 8192 106 -> 85
+//   input gradient   8192 x 4096 x 28672 1575 -> 1306    8192 x 14336 x 4096 796 -> 670     3003 x 2048 x 16384 208 -> 164
+//   weight gradient  28672 x 4096 x 8192 1690 -> 1447    128256 x 4096 x 4096 3788 -> 3286  16384 x 2048 x 3003 179 -> 154
+// (1310 - 1480 TFLOP/s for the large ones.)
 struct PairTile {
   static constexpr int kHalfBytes = 128 * BK * 2;                   // 128 x 64 of an operand
   static constexpr int kRingBytes = 12 * kHalfBytes;                // four stages of A and two of B, or six of A and one of B
